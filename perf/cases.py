@@ -397,9 +397,10 @@ def work(case):
 
 
 def tolerance(case):
-    # four times the largest error seen against `exact`; the accelerations and pressures of a forward run, second
-    # derivatives of an FP32 field that is smooth on the scale of the elements, carry the largest
-    return {"forward": {"rel": 1.4e-3}, "ocean": {"rel": 1.2e-3}, "gradient": {"rel": 1e-4},
+    # four times the largest difference seen between two orders of the sums over a step (elements taken in another
+    # order); the accelerations and pressures of a forward run, second derivatives of an FP32 field that is smooth on
+    # the scale of the elements, carry the largest
+    return {"forward": {"rel": 3.5e-3}, "ocean": {"rel": 1.4e-3}, "gradient": {"rel": 1e-4},
             "ocean_gradient": {"rel": 1e-4}, "smooth": {"rel": 2e-7, "max": 1e-5}}[case["kind"]]
 
 
