@@ -658,7 +658,7 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": TILE_TRAFFIC.get(traffic_key),
                      "traffic_source": TRAFFIC_SOURCE.get(traffic_key),
-                     "kernel": "k_elastic_tile", "kernel_ms": tile_ms, "shared_kernel_ms": shared_ms,
+                     "kernel": "k_elastic_rows", "kernel_ms": tile_ms, "shared_kernel_ms": shared_ms,
                      "fluid_kernels_ms": k_ms[:2] if coupled else None, "step_kernels_ms": k_ms[-1],
                      "algorithmic_bytes_per_launch": tile_bytes,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback"},

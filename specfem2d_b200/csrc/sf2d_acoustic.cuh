@@ -45,12 +45,19 @@ struct AcParams {
   const float *rmass;         // rmass_inverse_acoustic
   const uint8_t *free_mask;   // 1 on free-surface points
   const TileInfo *tiles;
+  // tiles by rows (sf2d_acoustic_lanes.cuh), per block of 32 elements, arrays are [block][q][lane]
+  const float4 *lgeo;         // xix, xiz, gammax, gammaz
+  const float *lfac;          // jacobian / rho formed in FP32
+  size_t nlane_q;             // their size
+  const uint32_t *lid;        // local ids of a row, and of the element's centre
+  const uint32_t *lphase;     // per element slot: assembly phase of position class k in byte k
+  // CPML tiles, per slot
   const uint16_t *lib;
-  const float4 *geo;          // xix, xiz, gammax, gammaz (tile slot order)
+  const float4 *geo;          // xix, xiz, gammax, gammaz
   const float *fac;           // jacobian / rho formed in FP32
   const int *sh_ids;
   float *partial;
-  const int *shp_off, *slot_pos;  // point-major partial sums, as in the solid kernels
+  const int *shp_off, *sh_slot;  // point-major partial sums, as in the solid kernels
   const int *edge_local;      // per tile (edge_off, edge_n): local point | free_mask bits << 16
   const int4 *bgroups;        // per tile (grp_off, grp_n): point, first idx, Stacey | coupling << 8, sources
   const int *bnd_idx;         // entries of each group
@@ -69,15 +76,17 @@ struct AcParams {
   const float4 *rec_geo;      // 25 per receiver: xix, xiz, gammax, gammaz
   const float *rec_rho;       // 25 per receiver
   double *seis;               // [irec][it][2] for all receivers of the run
-  int *d_step, *d_step_b;
+  int *d_step;
   int *d_status;
   int nstep_stf, nstage, nstep_seis, seismotype, use_trick, nrec;
   double cosrot, sinrot;
   float dt, dto2, dt2o2;
   float alpha[6], beta[6];
   int shared_begin, nshared;
-  int max_q, max_local;
+  int max_q, max_local;         // of the CPML tiles
+  int max_local_l, max_elems_l; // of the tiles by rows
   float hconst[60];           // hprime[25], hprimewgll[25], wxgll[5], wzgll[5]
+  float hsum[5];              // row sums of hprime
   // CPML: elements of slots >= pml_slot0 lie in the layer (see Params)
   int pml_slot0;
   const PmlSet *pml_sets;     // coefficient sets of the layer
@@ -100,14 +109,12 @@ struct AcParams {
   const int *pframe_base;
   int npframes;
   // adjoint sweep with kernel accumulation: forward chi frame = *kp_base - step;
-  // per element point (slot order) its fluid point, rho and kappa, and the
-  // sums of 1/rho grad(chi_adj) . grad(chi) dt and 1/kappa chi_adj_dd chi dt
+  // the sums of grad(chi_adj) . grad(chi) per element point ([block][q][lane]) and of
+  // chi_adj_dd chi per fluid point
   const float *kpframes;
   const int *kp_base;
-  const int *slot_ibool;
-  const float2 *slot_rk;
-  float2 *kl_ac;
-  int nslot_q, nglob_ac;
+  float *kl_ac, *kap_glob;
+  int nglob_ac;
 };
 
 // Scalar line helpers of the fluid kernel (as line_derivs / line_weighted of
@@ -143,45 +150,28 @@ __device__ __forceinline__ void line_weighted_ac(const AcParams &A, float *buf, 
 // chi_dot and chi_dot_dot before and after the forces
 constexpr uint8_t AC_FREE = 1, AC_EDGE = 2;
 
-// Shared-memory regions of one fluid tile, 16-byte aligned (pold and pml only
-// in CPML tiles).
+// Shared-memory regions of one fluid CPML tile, 16-byte aligned.
 struct AcSmem {
   size_t p, pd, acc, h, lib, mask, d1, d2, pold, od1, od2, pml, total;
 };
-__host__ __device__ inline AcSmem ac_smem_layout(int max_q, int max_local, bool pml = false) {
-  AcSmem L;
-  size_t o = 0;
-  L.p = o;
-  o = align16(o + static_cast<size_t>(max_local) * sizeof(float));
-  L.pd = o;
-  o = align16(o + static_cast<size_t>(max_local) * sizeof(float));
-  L.acc = o;
-  o = align16(o + static_cast<size_t>(max_local) * sizeof(float));
-  L.h = o;
-  o = align16(o + 64 * sizeof(float));
-  L.lib = o;
-  o = align16(o + static_cast<size_t>((max_q + 7) / 8 * 8) * sizeof(uint16_t));
-  L.mask = o;  // uint8 per local point: free surface / layer edge bits
-  o = align16(o + static_cast<size_t>(max_local));
+__host__ __device__ inline AcSmem ac_smem_layout(int max_q, int max_local) {
   const size_t qb = align16(static_cast<size_t>(max_q) * sizeof(float));
-  L.d1 = o;
-  o += qb;
-  L.d2 = o;
-  o += qb;
-  L.pold = o;
-  if (pml) o = align16(o + static_cast<size_t>(max_local) * sizeof(float));
-  L.od1 = o;
-  if (pml) o += qb;
-  L.od2 = o;
-  if (pml) o += qb;
-  L.pml = o;
-  if (pml) o += qb;
-  L.total = o;
+  const size_t lb = align16(static_cast<size_t>(max_local) * sizeof(float));
+  AcSmem L;
+  L.p = 0;
+  L.pd = L.p + lb;
+  L.acc = L.pd + lb;
+  L.h = L.acc + lb;
+  L.lib = L.h + align16(64 * sizeof(float));
+  L.mask = L.lib + align16(static_cast<size_t>((max_q + 7) / 8 * 8) * sizeof(uint16_t));  // uint8 per local point: free surface / layer edge bits
+  L.d1 = L.mask + align16(static_cast<size_t>(max_local));
+  L.d2 = L.d1 + qb;
+  L.pold = L.d2 + qb;
+  L.od1 = L.pold + lb;
+  L.od2 = L.od1 + qb;
+  L.pml = L.od2 + qb;
+  L.total = L.pml + qb;
   return L;
-}
-
-__device__ __forceinline__ void cp_async4(void *s, const void *g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr(s)), "l"(g) : "memory");
 }
 
 // Receiver in a fluid element (write_seismograms.F90:75-150): pressure
@@ -237,13 +227,65 @@ __device__ __forceinline__ void record_receiver_ac(const AcParams &A, int r, int
   out[1] = -A.sinrot * vx + A.cosrot * vz;
 }
 
+// Boundary terms, coupling and sources of a fluid tile: one thread per receiving
+// point, in the reference's order at that point.
+template <bool LDDRK>
+__device__ __forceinline__ void ac_boundary_terms(const AcParams &A, const TileInfo &ti, const float *s_pd, float *s_acc,
+                                                  int step, int stage, int tid, int nt) {
+  for (int gi = tid; gi < ti.grp_n; gi += nt) {
+    const int4 g = A.bgroups[ti.grp_off + gi];
+    const int l = g.x;
+    const int *ix = A.bnd_idx + g.y;
+    float acc = s_acc[l];
+    const int nst = g.z & 255, ncp = g.z >> 8;
+    for (int k = 0; k < nst; ++k) {
+      const float2 wr = A.st_wr[ix[k]];
+      acc = acc - s_pd[l] * wr.x / wr.y;
+    }
+    ix += nst;
+    // the solid's normal displacement; a negative source names the CPML entry
+    // ~src, whose displacement k_cpl_pml_fluid formed
+    for (int k = 0; k < ncp; ++k) {
+      const int q = ix[k];
+      const int ge = A.cpl_src[q];
+      const float4 nw = A.cpl_nw[q];
+      float2 u;
+      if (ge >= 0 && A.adjoint) {
+        const float2 a = A.a_el[ge];
+        u = make_float2(-a.x, -a.y);
+      } else if (ge >= 0) {
+        u = A.u_el[ge];
+        if (!LDDRK) {
+          const float2 v = A.v_el[ge], a = A.a_el[ge];
+          u.x = newmark_displ(u.x, v.x, a.x, A.dt, A.dt2o2);
+          u.y = newmark_displ(u.y, v.y, a.y, A.dt, A.dt2o2);
+        }
+      } else {
+        u = A.cpl_pml_u[~ge];
+      }
+      const float displ_n = u.x * nw.x + u.y * nw.y;
+      acc = acc + nw.z * displ_n;
+    }
+    ix += ncp;
+    for (int k = 0; k < g.w; ++k) {
+      const int q = ix[k];
+      const float f = step < A.nstep_stf
+                          ? A.stf[(static_cast<size_t>(A.src_id[q]) * A.nstep_stf + step) * A.nstage + stage]
+                          : 0.f;
+      const float2 sk = A.src_sk[q];
+      acc = acc + sk.x * f / sk.y;
+    }
+    s_acc[l] = acc;
+  }
+}
+
 // PML: the tiles of a CPML layer: mid-step chi + dt^2/4 chi_dot_dot, the
 // gradient and potential memory variables, the modified gradient and the
 // extra terms (pml_compute_memory_variables.f90:42-224,
 // pml_compute_accel_contribution.f90:42-180).  Tiles [tile0, tile0 + gridDim.x).
-template <int NT, bool LDDRK, bool PML = false>
-__global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
-    k_acoustic_tile(const AcParams A, int record_prev, int stage, int tile0) {
+template <int NT, bool LDDRK>
+__global__ void __launch_bounds__(NT, 768 / NT)
+    k_acoustic_pml_tile(const AcParams A, int stage, int tile0, int kstep) {
   extern __shared__ __align__(16) unsigned char smem[];
   const TileInfo &ti = A.tiles[tile0 + blockIdx.x];
   const int tid = threadIdx.x;
@@ -253,7 +295,7 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
   const int nq = ti.nelem * 25;
   const int ebase = ti.elem_base * 25;
   const int int_begin = ti.int_begin;
-  const AcSmem L = ac_smem_layout(A.max_q, A.max_local, PML);
+  const AcSmem L = ac_smem_layout(A.max_q, A.max_local);
   float *s_pold = reinterpret_cast<float *>(smem + L.pold);
   float *s_pml = reinterpret_cast<float *>(smem + L.pml);
   float *s_d1 = reinterpret_cast<float *>(smem + L.d1);
@@ -267,11 +309,9 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
   float *s_h = reinterpret_cast<float *>(smem + L.h);
   uint16_t *s_lib = reinterpret_cast<uint16_t *>(smem + L.lib);
 
-  const int step = *A.d_step;
-  if (blockIdx.x == 0 && tid == 0) *A.d_step_b = step;
   // fluid receivers are recorded by k_acoustic_receivers after each step: their
   // double-precision gradient would hold registers through the whole tile
-  (void)record_prev;
+  const int step = *A.d_step + kstep;
 
   // 1. loads
   {
@@ -304,7 +344,7 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
     if (!LDDRK) {
       const float pdd = s_acc[l];
       // mid-step potential (update_displacement_Newmark.F90:374-380)
-      if (PML) s_pold[l] = static_cast<float>(static_cast<double>(p) + A.h_old * static_cast<double>(pdd));
+      s_pold[l] = static_cast<float>(static_cast<double>(p) + A.h_old * static_cast<double>(pdd));
       p = newmark_displ(p, pd, pdd, dt, dt2o2);
       pd = newmark_veloc(pd, pdd, dto2);
     }
@@ -321,59 +361,14 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
       const uint8_t m = static_cast<uint8_t>(v >> 16);
       s_p[l] = 0.f;
       s_pd[l] = 0.f;
-      if (PML && !LDDRK && (m & AC_EDGE)) s_pold[l] = 0.f;  // the layer's edge (pml_boundary_acoustic)
+      if (!LDDRK && (m & AC_EDGE)) s_pold[l] = 0.f;  // the layer's edge (pml_boundary_acoustic)
       s_mask[l] = m;
     }
     __syncthreads();
   }
 
-  // 3. boundary terms, coupling and sources: one thread per receiving point,
-  //    in the reference's order at that point
-  for (int gi = tid; gi < ti.grp_n; gi += NT) {
-    const int4 g = A.bgroups[ti.grp_off + gi];
-    const int l = g.x;
-    const int *ix = A.bnd_idx + g.y;
-    float acc = s_acc[l];
-    const int nst = g.z & 255, ncp = g.z >> 8;
-    for (int k = 0; k < nst; ++k) {
-      const float2 wr = A.st_wr[ix[k]];
-      acc = acc - s_pd[l] * wr.x / wr.y;
-    }
-    ix += nst;
-    // the solid's normal displacement; a negative source names the CPML entry
-    // ~src, whose displacement k_cpl_pml_fluid formed
-    for (int k = 0; k < ncp; ++k) {
-      const int q = ix[k];
-      const int ge = A.cpl_src[q];
-      const float4 nw = A.cpl_nw[q];
-      float2 u;
-      if (ge >= 0 && A.adjoint) {
-        const float2 a = A.a_el[ge];
-        u = make_float2(-a.x, -a.y);
-      } else if (ge >= 0) {
-        u = A.u_el[ge];
-        if (!LDDRK) {
-          const float2 v = A.v_el[ge], a = A.a_el[ge];
-          u.x = newmark_displ(u.x, v.x, a.x, dt, dt2o2);
-          u.y = newmark_displ(u.y, v.y, a.y, dt, dt2o2);
-        }
-      } else {
-        u = A.cpl_pml_u[~ge];
-      }
-      const float displ_n = u.x * nw.x + u.y * nw.y;
-      acc = acc + nw.z * displ_n;
-    }
-    ix += ncp;
-    for (int k = 0; k < g.w; ++k) {
-      const int q = ix[k];
-      const float f = step < A.nstep_stf
-                          ? A.stf[(static_cast<size_t>(A.src_id[q]) * A.nstep_stf + step) * A.nstage + stage]
-                          : 0.f;
-      const float2 sk = A.src_sk[q];
-      acc = acc + sk.x * f / sk.y;
-    }
-    s_acc[l] = acc;
-  }
+  // 3. boundary terms, coupling and sources
+  ac_boundary_terms<LDDRK>(A, ti, s_pd, s_acc, step, stage, tid, NT);
 
   // the first point's geometry and J/rho are requested now (see the solid kernel)
   float4 g_next = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -395,7 +390,7 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
     const uint16_t *le = s_lib + 25 * e + a0;
     const int o = 25 * e + a0;
     line_derivs_ac(A, s_p, le, st, (r < 5 ? s_d1 : s_d2) + o);
-    if (PML && !LDDRK) line_derivs_ac(A, s_pold, le, st, (r < 5 ? s_od1 : s_od2) + o);
+    if (!LDDRK) line_derivs_ac(A, s_pold, le, st, (r < 5 ? s_od1 : s_od2) + o);
   }
   __syncthreads();
 
@@ -419,49 +414,47 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
     }
     float dxl = dxi * g4.x + dgam * g4.z;
     float dzl = dxi * g4.y + dgam * g4.w;
-    if (PML) {
-      const int ps = ebase + f - 25 * A.pml_slot0;
-      const PmlSet &c = A.pml_sets[A.pml_set_idx[ps]];
-      float dxl_o = 0.f, dzl_o = 0.f;
-      if (!LDDRK) {
-        const float oxi = s_od1[f], og = s_od2[f];
-        dxl_o = oxi * g4.x + og * g4.z;
-        dzl_o = oxi * g4.y + og * g4.w;
-      }
-      const PmlConv &cax = c.cax, &caz = c.caz, &cbx = c.cbx, &cbz = c.cbz;
-      const PmlLik &zx = c.zx, &xz = c.xz;  // poles (alpha_z, beta_x) and (alpha_x, beta_z)
-      float2 rx = A.pml_rm[3 * ps], rz = A.pml_rm[3 * ps + 1], rp = A.pml_rm[3 * ps + 2];
-      float2 lx = make_float2(0.f, 0.f), lz = lx, lp = lx;
-      if (LDDRK) {
-        lx = A.pml_rm_l[3 * ps];
-        lz = A.pml_rm_l[3 * ps + 1];
-        lp = A.pml_rm_l[3 * ps + 2];
-      }
-      const float al = A.alpha[stage], be = A.beta[stage];
-      pml_update<LDDRK>(rx.x, lx.x, caz, c.az, dxl, dxl_o, al, be, dt);
-      pml_update<LDDRK>(rx.y, lx.y, cbx, c.bx, dxl, dxl_o, al, be, dt);
-      pml_update<LDDRK>(rz.x, lz.x, cax, c.ax, dzl, dzl_o, al, be, dt);
-      pml_update<LDDRK>(rz.y, lz.y, cbz, c.bz, dzl, dzl_o, al, be, dt);
-      dxl = static_cast<float>(zx.A0 * dxl + zx.A1 * rx.x + zx.A2 * rx.y);
-      dzl = static_cast<float>(xz.A0 * dzl + xz.A1 * rz.x + xz.A2 * rz.y);
-      // the layer's terms at this point (pml_compute_accel_contribution.f90:42-180)
-      const PmlL &Lc = c.l;  // poles alpha_x, alpha_z
-      const int lq = le[q];
-      const float pq = s_p[lq], pdq = s_pd[lq];
-      const float po = LDDRK ? 0.f : s_pold[lq];
-      pml_update<LDDRK>(rp.x, lp.x, cax, c.ax, pq, po, al, be, dt);
-      pml_update<LDDRK>(rp.y, lp.y, caz, c.az, pq, po, al, be, dt);
-      const float wwf = s_h[50 + i] * s_h[55 + j] * A.pml_jk[ps];
-      s_pml[f] = static_cast<float>(static_cast<double>(wwf) *
-                                    (Lc.A1 * pdq + Lc.A2 * pq + Lc.A3 * rp.x + Lc.A4 * rp.y));
-      A.pml_rm[3 * ps] = rx;
-      A.pml_rm[3 * ps + 1] = rz;
-      A.pml_rm[3 * ps + 2] = rp;
-      if (LDDRK) {
-        A.pml_rm_l[3 * ps] = lx;
-        A.pml_rm_l[3 * ps + 1] = lz;
-        A.pml_rm_l[3 * ps + 2] = lp;
-      }
+    const int ps = ebase + f - 25 * A.pml_slot0;
+    const PmlSet &c = A.pml_sets[A.pml_set_idx[ps]];
+    float dxl_o = 0.f, dzl_o = 0.f;
+    if (!LDDRK) {
+      const float oxi = s_od1[f], og = s_od2[f];
+      dxl_o = oxi * g4.x + og * g4.z;
+      dzl_o = oxi * g4.y + og * g4.w;
+    }
+    const PmlConv &cax = c.cax, &caz = c.caz, &cbx = c.cbx, &cbz = c.cbz;
+    const PmlLik &zx = c.zx, &xz = c.xz;  // poles (alpha_z, beta_x) and (alpha_x, beta_z)
+    float2 rx = A.pml_rm[3 * ps], rz = A.pml_rm[3 * ps + 1], rp = A.pml_rm[3 * ps + 2];
+    float2 lx = make_float2(0.f, 0.f), lz = lx, lp = lx;
+    if (LDDRK) {
+      lx = A.pml_rm_l[3 * ps];
+      lz = A.pml_rm_l[3 * ps + 1];
+      lp = A.pml_rm_l[3 * ps + 2];
+    }
+    const float al = A.alpha[stage], be = A.beta[stage];
+    pml_update<LDDRK>(rx.x, lx.x, caz, c.az, dxl, dxl_o, al, be, dt);
+    pml_update<LDDRK>(rx.y, lx.y, cbx, c.bx, dxl, dxl_o, al, be, dt);
+    pml_update<LDDRK>(rz.x, lz.x, cax, c.ax, dzl, dzl_o, al, be, dt);
+    pml_update<LDDRK>(rz.y, lz.y, cbz, c.bz, dzl, dzl_o, al, be, dt);
+    dxl = static_cast<float>(zx.A0 * dxl + zx.A1 * rx.x + zx.A2 * rx.y);
+    dzl = static_cast<float>(xz.A0 * dzl + xz.A1 * rz.x + xz.A2 * rz.y);
+    // the layer's terms at this point (pml_compute_accel_contribution.f90:42-180)
+    const PmlL &Lc = c.l;  // poles alpha_x, alpha_z
+    const int lq = le[q];
+    const float pq = s_p[lq], pdq = s_pd[lq];
+    const float po = LDDRK ? 0.f : s_pold[lq];
+    pml_update<LDDRK>(rp.x, lp.x, cax, c.ax, pq, po, al, be, dt);
+    pml_update<LDDRK>(rp.y, lp.y, caz, c.az, pq, po, al, be, dt);
+    const float wwf = s_h[50 + i] * s_h[55 + j] * A.pml_jk[ps];
+    s_pml[f] = static_cast<float>(static_cast<double>(wwf) *
+                                  (Lc.A1 * pdq + Lc.A2 * pq + Lc.A3 * rp.x + Lc.A4 * rp.y));
+    A.pml_rm[3 * ps] = rx;
+    A.pml_rm[3 * ps + 1] = rz;
+    A.pml_rm[3 * ps + 2] = rp;
+    if (LDDRK) {
+      A.pml_rm_l[3 * ps] = lx;
+      A.pml_rm_l[3 * ps + 1] = lz;
+      A.pml_rm_l[3 * ps + 2] = lp;
     }
     s_d1[f] = fac * (g4.x * dxl + g4.y * dzl);
     s_d2[f] = fac * (g4.z * dxl + g4.w * dzl);
@@ -488,70 +481,58 @@ __global__ void __launch_bounds__(NT, PML ? 768 / NT : 1536 / NT)
       const int j = FIXQ ? j0 : q / 5;
       const int i = FIXQ ? i0 : q - 5 * j;
       const int l = s_lib[f];
-      float acc = s_acc[l] - (s_h[55 + j] * s_d1[f] + s_h[50 + i] * s_d2[f]);
-      if (PML) acc = acc - s_pml[f];
-      s_acc[l] = acc;
+      s_acc[l] = s_acc[l] - (s_h[55 + j] * s_d1[f] + s_h[50 + i] * s_d2[f]) - s_pml[f];
     }
     cb = ce;
     __syncthreads();
   }
 
-  // 6. mass, corrector or LDDRK update, free surface, write-back (each
-  //    point's rmass, mask or slot requested one iteration ahead)
+  // 6. mass, corrector or LDDRK update, free surface, write-back (each point's
+  //    rmass requested one iteration ahead)
   bool bad = false;
   float rm_next = 0.f;
-  int sp_next = 0;
-  if (tid < n_int)
-    rm_next = A.rmass[int_begin + tid];
-  else if (tid < nl)
-    sp_next = A.slot_pos[ti.sh_off + tid - n_int];
+  if (tid < n_int) rm_next = A.rmass[int_begin + tid];
   for (int l = tid; l < nl; l += NT) {
     const float acc = s_acc[l];
     const float rm = rm_next;
-    const uint8_t fm = s_mask[l];
-    const int sp = sp_next;
-    if (l + NT < n_int) {
-      rm_next = A.rmass[int_begin + l + NT];
-    } else if (l + NT < nl) {
-      sp_next = A.slot_pos[ti.sh_off + l + NT - n_int];
+    if (l + NT < n_int) rm_next = A.rmass[int_begin + l + NT];
+    if (l >= n_int) {
+      A.partial[A.sh_slot[ti.sh_off + l - n_int]] = acc;
+      continue;
     }
-    if (l < n_int) {
-      const int g = int_begin + l;
-      float pdd = acc * rm;
-      float pd = s_pd[l], p = s_p[l];
-      if (!LDDRK) {
-        pd = newmark_veloc(pd, pdd, dto2);
-      } else {
-        const float al = A.alpha[stage], be = A.beta[stage];
-        float pdl = A.pdL[g], pl = A.pL[g];
-        pdl = al * pdl + dt * pdd;
-        pl = al * pl + dt * pd;
-        pd = pd + be * pdl;
-        p = p + be * pl;
-        A.pdL[g] = pdl;
-        A.pL[g] = pl;
-      }
-      if (fm) {
-        p = 0.f;
-        pd = 0.f;
-        pdd = 0.f;
-      }
-      A.p[g] = p;
-      A.pd[g] = pd;
-      A.pdd[g] = pdd;
-      if (PML && !LDDRK && A.pold) A.pold[g] = s_pold[l];
-      bad |= !(fabsf(p) < 1e25f);
+    const int g = int_begin + l;
+    float pdd = acc * rm;
+    float pd = s_pd[l], p = s_p[l];
+    if (!LDDRK) {
+      pd = newmark_veloc(pd, pdd, dto2);
     } else {
-      A.partial[sp] = acc;
+      const float al = A.alpha[stage], be = A.beta[stage];
+      float pdl = A.pdL[g], pl = A.pL[g];
+      pdl = al * pdl + dt * pdd;
+      pl = al * pl + dt * pd;
+      pd = pd + be * pdl;
+      p = p + be * pl;
+      A.pdL[g] = pdl;
+      A.pL[g] = pl;
     }
+    if (s_mask[l]) {
+      p = 0.f;
+      pd = 0.f;
+      pdd = 0.f;
+    }
+    A.p[g] = p;
+    A.pd[g] = pd;
+    A.pdd[g] = pdd;
+    if (!LDDRK && A.pold) A.pold[g] = s_pold[l];
+    bad |= !(fabsf(p) < 1e25f);
   }
   if (bad) *A.d_status = 1;
 }
 
 template <bool LDDRK>
-__global__ void __launch_bounds__(SHARED_NT) k_acoustic_shared(const AcParams A, int stage, int last_stage) {
+__global__ void __launch_bounds__(SHARED_NT) k_acoustic_shared(const AcParams A, int stage, int kstep) {
   const int s = blockIdx.x * SHARED_NT + threadIdx.x;
-  const int step = *A.d_step_b;
+  const int step = *A.d_step + kstep;
   if (s < A.nshared) {
     const int g = A.shared_begin + s;
     float p = A.p[g], pd = A.pd[g];
@@ -592,9 +573,17 @@ __global__ void __launch_bounds__(SHARED_NT) k_acoustic_shared(const AcParams A,
     A.p[g] = p;
     A.pd[g] = pd;
     A.pdd[g] = pdd;
+    if (A.pframes) {
+      const int fi = step - *A.pframe_base;
+      if (fi >= 0 && fi < A.npframes) A.pframes[static_cast<size_t>(fi) * A.nglob_ac + g] = p;
+    }
+    if (A.kap_glob) {
+      const int fi = *A.kp_base - step;
+      if (fi >= 0 && fi < A.npframes)
+        A.kap_glob[g] = A.kap_glob[g] + pdd * A.kpframes[static_cast<size_t>(fi) * A.nglob_ac + g];
+    }
     if (!(fabsf(p) < 1e25f)) *A.d_status = 1;
   }
-  if (last_stage && blockIdx.x == 0 && threadIdx.x == 0) *A.d_step = step + 1;
 }
 
 // Coupling entries next to a CPML layer, one thread per entry, once per step
@@ -664,55 +653,14 @@ __global__ void k_cpl_pml_solid(const CplPml C, const float *p, const float *pd,
                                   c[2] * static_cast<double>(pot) + c[3] * static_cast<double>(r)));
 }
 
-// records the step before *d_step for every fluid receiver (launched after the
-// last stage of every step)
-static __global__ void k_acoustic_receivers(const AcParams A) {
+// records step *d_step + kstep for every fluid receiver (launched after the last
+// stage of every step)
+static __global__ void k_acoustic_receivers(const AcParams A, int kstep) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < A.nrec) record_receiver_ac(A, r, *A.d_step - 1);
+  if (r < A.nrec) record_receiver_ac(A, r, *A.d_step + kstep);
 }
 
-// After a finished step (*d_step already advanced): chi into its frame when the
-// frame lies in [0, npframes).
-static __global__ void k_fluid_frame(const AcParams A) {
-  const int fi = (*A.d_step - 1) - *A.pframe_base;
-  if (fi < 0 || fi >= A.npframes) return;
-  float *dst = A.pframes + static_cast<size_t>(fi) * A.nglob_ac;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < A.nglob_ac; g += gridDim.x * blockDim.x) dst[g] = A.p[g];
-}
-
-// compute_kernels_ac (compute_kernels.f90:293-449; the GPU form,
-// compute_kernels_acoustic_cuda in src/gpu/compute_kernels_cuda.cu), after a
-// finished adjoint step: at every fluid element point the gradients of the
-// adjoint chi and of the forward chi of the paired frame (derivative lines in
-// FP32, the mapping applied in double and stored in FP32), and
-//   sum.x += 1/rho (grad chi_adj . grad chi) dt,  sum.y += 1/kappa chi_adj_dd chi dt.
-static __global__ void k_fluid_kernels(const AcParams A) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= A.nslot_q) return;
-  const int fi = *A.kp_base - (*A.d_step - 1);
-  if (fi < 0 || fi >= A.npframes) return;  // no paired frame: nothing accumulates
-  const float *b = A.kpframes + static_cast<size_t>(fi) * A.nglob_ac;
-  const int e0 = q - q % 25, i = q % 5, j = (q % 25) / 5;
-  float t1 = 0.f, t2 = 0.f, b1 = 0.f, b2 = 0.f;
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    const int gr = A.slot_ibool[e0 + j * 5 + k], gc = A.slot_ibool[e0 + k * 5 + i];
-    t1 = t1 + A.p[gr] * A.hconst[5 * i + k];
-    b1 = b1 + b[gr] * A.hconst[5 * i + k];
-    t2 = t2 + A.p[gc] * A.hconst[5 * j + k];
-    b2 = b2 + b[gc] * A.hconst[5 * j + k];
-  }
-  const float4 gm = A.geo[q];
-  const float ax = static_cast<float>(static_cast<double>(t1) * gm.x + static_cast<double>(t2) * gm.z);
-  const float az = static_cast<float>(static_cast<double>(t1) * gm.y + static_cast<double>(t2) * gm.w);
-  const float bx = static_cast<float>(static_cast<double>(b1) * gm.x + static_cast<double>(b2) * gm.z);
-  const float bz = static_cast<float>(static_cast<double>(b1) * gm.y + static_cast<double>(b2) * gm.w);
-  const int g = A.slot_ibool[q];
-  const float2 rk = A.slot_rk[q];
-  float2 s = A.kl_ac[q];
-  s.x = s.x + 1.f / rk.x * (ax * bx + az * bz) * A.dt;
-  s.y = s.y + 1.f / rk.y * A.pdd[g] * b[g] * A.dt;
-  A.kl_ac[q] = s;
-}
+// after n steps: the step counter
+static __global__ void k_acoustic_advance(const AcParams A, int n) { *A.d_step += n; }
 
 }  // namespace sf2d

@@ -10,7 +10,7 @@
 #include <string>
 #include <vector>
 
-#include "sf2d_acoustic.cuh"
+#include "sf2d_acoustic_rows.cuh"
 #include "sf2d_b200.h"
 #include "sf2d_coupled.h"
 #include "sf2d_kernels.cuh"
@@ -44,13 +44,12 @@ __global__ void k_scatter_f2(const float2 *src, const int *map, float2 *dst, int
 
 using AcTileFn = void (*)(AcParams, int, int, int);
 
-template <bool PML>
-AcTileFn pick_ac_tile(int nt, bool lddrk) {
+AcTileFn pick_ac_pml_tile(int nt, bool lddrk) {
   switch (nt) {
-    case 128: return lddrk ? sf2d::k_acoustic_tile<128, true, PML> : sf2d::k_acoustic_tile<128, false, PML>;
-    case 250: return lddrk ? sf2d::k_acoustic_tile<250, true, PML> : sf2d::k_acoustic_tile<250, false, PML>;
-    case 512: return lddrk ? sf2d::k_acoustic_tile<512, true, PML> : sf2d::k_acoustic_tile<512, false, PML>;
-    default: return lddrk ? sf2d::k_acoustic_tile<256, true, PML> : sf2d::k_acoustic_tile<256, false, PML>;
+    case 128: return lddrk ? sf2d::k_acoustic_pml_tile<128, true> : sf2d::k_acoustic_pml_tile<128, false>;
+    case 250: return lddrk ? sf2d::k_acoustic_pml_tile<250, true> : sf2d::k_acoustic_pml_tile<250, false>;
+    case 512: return lddrk ? sf2d::k_acoustic_pml_tile<512, true> : sf2d::k_acoustic_pml_tile<512, false>;
+    default: return lddrk ? sf2d::k_acoustic_pml_tile<256, true> : sf2d::k_acoustic_pml_tile<256, false>;
   }
 }
 
@@ -94,6 +93,8 @@ struct sf2d_coupled {
   int pml_tile0 = 0;
   size_t pml_smem = 0;
   size_t smem = 0;
+  int lane_nt = 32;             // threads per CTA of the tiles by rows
+  std::vector<int> slot_lane;   // tiles by rows: slot -> the element's lane
   int nt = 256, nstage = 1, nglob = 0, nrec_total = 0, nstep = 0, steps_done = 0;
   size_t npml_q = 0;  // GLL points of the fluid CPML elements
   bool lddrk = false;
@@ -146,29 +147,27 @@ struct sf2d_coupled {
   // the fluid's CPML tiles beside the others, as the solid's (sf2d_solver::launch_tile)
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  void launch_ac_tile(bool record_prev, int stage) {
-    const int rp = record_prev ? 1 : 0;
+  void launch_ac_tile(int stage, int kstep) {
     cudaStream_t s = stream();
     if (side) {
       cudaEventRecord(ev_fork, s);
       cudaStreamWaitEvent(side, ev_fork, 0);
-      pml_fn<<<T.ntiles - pml_tile0, nt, pml_smem, side>>>(A, rp, stage, pml_tile0);
+      pml_fn<<<T.ntiles - pml_tile0, nt, pml_smem, side>>>(A, stage, pml_tile0, kstep);
       cudaEventRecord(ev_join, side);
-      tile_fn<<<pml_tile0, nt, smem, s>>>(A, rp, stage, 0);
+      tile_fn<<<pml_tile0, lane_nt, smem, s>>>(A, stage, 0, kstep);
       cudaStreamWaitEvent(s, ev_join, 0);
       return;
     }
-    if (pml_tile0 > 0) tile_fn<<<pml_tile0, nt, smem, s>>>(A, rp, stage, 0);
-    if (pml_tile0 < T.ntiles)
-      (pml_fn ? pml_fn : tile_fn)<<<T.ntiles - pml_tile0, nt, pml_fn ? pml_smem : smem, s>>>(A, rp, stage, pml_tile0);
+    if (pml_tile0 > 0) tile_fn<<<pml_tile0, lane_nt, smem, s>>>(A, stage, 0, kstep);
+    if (pml_tile0 < T.ntiles) pml_fn<<<T.ntiles - pml_tile0, nt, pml_smem, s>>>(A, stage, pml_tile0, kstep);
   }
-  void launch_ac_shared(int stage) {
-    const int nb = std::max(1, (A.nshared + sf2d::SHARED_NT - 1) / sf2d::SHARED_NT);
-    const int last = stage == nstage - 1 ? 1 : 0;
+  void launch_ac_shared(int stage, int kstep) {
+    if (A.nshared == 0) return;
+    const int nb = (A.nshared + sf2d::SHARED_NT - 1) / sf2d::SHARED_NT;
     if (lddrk)
-      sf2d::k_acoustic_shared<true><<<nb, sf2d::SHARED_NT, 0, stream()>>>(A, stage, last);
+      sf2d::k_acoustic_shared<true><<<nb, sf2d::SHARED_NT, 0, stream()>>>(A, stage, kstep);
     else
-      sf2d::k_acoustic_shared<false><<<nb, sf2d::SHARED_NT, 0, stream()>>>(A, stage, last);
+      sf2d::k_acoustic_shared<false><<<nb, sf2d::SHARED_NT, 0, stream()>>>(A, stage, kstep);
   }
   void launch_cpl_fluid(int stage) {
     if (cpl_fluid.n == 0) return;
@@ -198,71 +197,63 @@ struct sf2d_coupled {
   cudaStream_t early = nullptr;
   cudaEvent_t ev_early_fork = nullptr, ev_early_join = nullptr;
   bool rec_pending = false;
-  void launch_ac_receivers() {
+  void launch_ac_receivers(int kstep) {
     if (A.nrec <= 0) return;
     const int nb = (A.nrec + 127) / 128;
     if (side) {
       cudaEventRecord(ev_rec, stream());
       cudaStreamWaitEvent(side, ev_rec, 0);
-      sf2d::k_acoustic_receivers<<<nb, 128, 0, side>>>(A);
+      sf2d::k_acoustic_receivers<<<nb, 128, 0, side>>>(A, kstep);
       cudaEventRecord(ev_rec_done, side);
       rec_pending = true;
     } else {
-      sf2d::k_acoustic_receivers<<<nb, 128, 0, stream()>>>(A);
+      sf2d::k_acoustic_receivers<<<nb, 128, 0, stream()>>>(A, kstep);
     }
   }
   void join_ac_receivers() {
     if (rec_pending) cudaStreamWaitEvent(stream(), ev_rec_done, 0);
     rec_pending = false;
   }
-  // after a finished fluid step: its chi frame (segment recomputation) and the
-  // fluid kernel sums (adjoint sweep), when the run keeps them
-  void launch_fluid_post() {
-    if (A.pframes) sf2d::k_fluid_frame<<<std::min(1184, (nglob + 255) / 256), 256, 0, stream()>>>(A);
-    if (A.kl_ac) sf2d::k_fluid_kernels<<<(A.nslot_q + 127) / 128, 128, 0, stream()>>>(A);
-  }
-  void launch_step(bool record_prev) {
+  // the k-th step of a chunk
+  void launch_step(int k) {
     if (adjoint) {
       // kernel runs switch the order: the whole solid step, then the fluid step
       // (iterate_time.F90:298-327); Newmark, no CPML, no side streams
       if (el) {
-        el->launch_tile(record_prev, 0, 0);
-        el->launch_shared(0);
+        el->launch_tile(k > 0, 0, 0, k);
+        el->launch_shared(0, k);
       }
-      launch_ac_tile(record_prev, 0);
-      launch_ac_shared(0);
-      launch_ac_receivers();
-      launch_fluid_post();
+      launch_ac_tile(0, k);
+      launch_ac_shared(0, k);
+      launch_ac_receivers(k);
       return;
     }
     for (int st = 0; st < nstage; ++st) {
-      const bool split = el && early && el->late_tile0 > 0;
+      const bool split = el && early && el->late_tile0 > 0, record_prev = k > 0 && st == 0;
       if (split) {
         cudaEventRecord(ev_early_fork, stream());
         cudaStreamWaitEvent(early, ev_early_fork, 0);
-        el->launch_early(early, record_prev && st == 0, st);
+        el->launch_early(early, record_prev, st, k);
         cudaEventRecord(ev_early_join, early);
       }
       launch_cpl_fluid(st);
       join_ac_receivers();
-      launch_ac_tile(record_prev && st == 0, st);
-      launch_ac_shared(st);
-      if (st == nstage - 1) {
-        launch_ac_receivers();
-        launch_fluid_post();
-      }
+      launch_ac_tile(st, k);
+      launch_ac_shared(st, k);
+      if (st == nstage - 1) launch_ac_receivers(k);
       launch_cpl_solid(st);
       if (el) {
-        el->launch_tile(record_prev && st == 0, st, split ? el->late_tile0 : 0);
+        el->launch_tile(record_prev, st, split ? el->late_tile0 : 0, k);
         if (split) cudaStreamWaitEvent(stream(), ev_early_join, 0);
-        el->launch_shared(st);
+        el->launch_shared(st, k);
       }
     }
   }
   int launch_chunk(int n) {
-    for (int k = 0; k < n; ++k) launch_step(k > 0);
+    for (int k = 0; k < n; ++k) launch_step(k);
     join_ac_receivers();
-    if (el) el->launch_receivers();
+    sf2d::k_acoustic_advance<<<1, 1, 0, stream()>>>(A, n);
+    if (el) el->launch_advance(n);
     SF2D_CUDA(cudaGetLastError());
     return SF2D_OK;
   }
@@ -419,24 +410,65 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   int rc = 0;
 
   // ---- fluid tiling and per-slot data
-  const int te = ad->tile_elems > 0 ? ad->tile_elems : 32;
+  if (ad->tile_elems > 256) return fail(SF2D_ERR_INVALID, "fluid tiling: tile_elems must be in [1, 256]");
+  // five threads an element: 128 elements fit a block and its registers
+  const int te = std::min(ad->tile_elems > 0 ? ad->tile_elems : 32, 128);
   // the fluid layer's tiles are a quarter of the size: there are few of them
   // (one wave), so the shorter per-tile latency sets the layer kernel's time
-  const int group_te[2] = {te, std::max(4, te / 4)};
+  const int group_te[2] = {te, std::max(4, (ad->tile_elems > 0 ? ad->tile_elems : 32) / 4)};
   std::string err = build_tiling(ad->nspec, ad->nglob, ad->ibool, ad->centroid_xz, te, C->T,
-                                 pml_ac ? group.data() : nullptr, pml_ac ? 2 : 1, pml_ac ? group_te : nullptr);
+                                 pml_ac ? group.data() : nullptr, pml_ac ? 2 : 1, pml_ac ? group_te : nullptr, 1);
   if (!err.empty()) return fail(SF2D_ERR_INVALID, "fluid tiling: " + err);
   const Tiling &T = C->T;
   C->pml_tile0 = pml_ac ? T.group_tile_begin[1] : T.ntiles;
   const int pml_slot0 = C->pml_tile0 < T.ntiles ? T.tiles[C->pml_tile0].elem_base : ad->nspec;
-  const size_t nq = static_cast<size_t>(ad->nspec) * NGLL2;
-  std::vector<float4> geo(nq);
-  std::vector<float> fac(nq);
-  for (int s = 0; s < ad->nspec; ++s) {
-    const size_t src = static_cast<size_t>(T.elem_order[s]) * NGLL2;
-    for (int q = 0; q < NGLL2; ++q) {
-      geo[s * NGLL2 + q] = make_float4(ad->xix[src + q], ad->xiz[src + q], ad->gammax[src + q], ad->gammaz[src + q]);
-      fac[s * NGLL2 + q] = ad->jacobian[src + q] / ad->rhostore[src + q];  // deriv(6) = J / rho in FP32
+  AcParams &A = C->A;
+  std::vector<TileInfo> tiles = T.tiles;
+  // tiles by rows
+  C->slot_lane.resize(pml_slot0);
+  const size_t nlane_q = static_cast<size_t>(T.nlanes) * NGLL;
+  std::vector<float> lfac(nlane_q, 0.f);
+  std::vector<float4> lgeo(nlane_q, make_float4(0.f, 0.f, 0.f, 0.f));
+  std::vector<uint32_t> lid(static_cast<size_t>(T.nlanes) * 3, 0);
+  std::vector<uint32_t> lphase(T.phases.begin(), T.phases.begin() + pml_slot0);
+  for (int t = 0; t < C->pml_tile0; ++t) {
+    const TileInfo &ti = tiles[t];
+    C->lane_nt = std::max(C->lane_nt, (5 * ti.nelem + 31) / 32 * 32);
+    A.max_elems_l = std::max(A.max_elems_l, ti.nelem);
+    A.max_local_l = std::max(A.max_local_l, ti.n_int + ti.n_sh);
+    for (int k = 0; k < ti.nelem; ++k) {
+      const int s = ti.elem_base + k;
+      C->slot_lane[s] = ti.lane0 + 5 * k;
+      const size_t src = static_cast<size_t>(T.elem_order[s]) * NGLL2;
+      const uint16_t *lib = &T.lib[static_cast<size_t>(ti.lib_off) + static_cast<size_t>(k) * NGLL2];
+      for (int j = 0; j < NGLL; ++j) {
+        const int r = C->slot_lane[s] + j;
+        const size_t blk = static_cast<size_t>(r / 32);
+        for (int i = 0; i < NGLL; ++i) {
+          const size_t p = src + NGLL * j + i, dst = (blk * NGLL + i) * 32 + r % 32;
+          lgeo[dst] = make_float4(ad->xix[p], ad->xiz[p], ad->gammax[p], ad->gammaz[p]);
+          lfac[dst] = ad->jacobian[p] / ad->rhostore[p];  // deriv(6) = J / rho in FP32
+        }
+        const uint16_t *l = lib + NGLL * j;
+        lid[blk * 96 + r % 32] = l[0] | static_cast<uint32_t>(l[1]) << 16;
+        lid[blk * 96 + 32 + r % 32] = l[2] | static_cast<uint32_t>(l[3]) << 16;
+        lid[blk * 96 + 64 + r % 32] = l[4] | static_cast<uint32_t>(lib[12]) << 16;
+      }
+    }
+  }
+  // CPML tiles: per slot (all slots, so that the layer's are where its kernel looks)
+  std::vector<float4> geo;
+  std::vector<float> fac;
+  if (pml_ac) {
+    const size_t nq = static_cast<size_t>(ad->nspec) * NGLL2;
+    geo.resize(nq);
+    fac.resize(nq);
+    for (int s = pml_slot0; s < ad->nspec; ++s) {
+      const size_t src = static_cast<size_t>(T.elem_order[s]) * NGLL2;
+      for (int q = 0; q < NGLL2; ++q) {
+        geo[s * NGLL2 + q] = make_float4(ad->xix[src + q], ad->xiz[src + q], ad->gammax[src + q], ad->gammaz[src + q]);
+        fac[s * NGLL2 + q] = ad->jacobian[src + q] / ad->rhostore[src + q];  // deriv(6) = J / rho in FP32
+      }
     }
   }
   std::vector<float> rmass(ad->nglob);
@@ -463,7 +495,6 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
       const int g = ad->ibool[static_cast<size_t>(e) * NGLL2 + q];
       if (glob_tile[g] < 0) glob_tile[g] = T.elem_tile[e];
     }
-  std::vector<TileInfo> tiles = T.tiles;
   std::vector<std::vector<int>> st_t(T.ntiles), cpl_t(T.ntiles), src_t(T.ntiles), rec_t(T.ntiles);
   for (int k = 0; k < ad->nstacey; ++k) st_t[glob_tile[ad->st_iglob[k]]].push_back(k);
   for (int k = 0; k < cp->ncpl_ac; ++k) cpl_t[glob_tile[cp->cpl_ac_point[k]]].push_back(k);
@@ -531,17 +562,13 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
     }
     tiles[t].rec_n = static_cast<int>(rec_id.size()) - tiles[t].rec_off;
   }
-  for (const TileInfo &t : tiles)
-    if (t.rec_n > C->nt) return fail(SF2D_ERR_INVALID, "more fluid receivers in one tile than threads per CTA");
-  std::vector<int> slot_pos(T.shp_slots.size());
-  for (size_t k = 0; k < T.shp_slots.size(); ++k) slot_pos[T.shp_slots[k]] = static_cast<int>(k);
   // per tile: the local points on the free surface or a layer's outer edge, with their bits
   std::vector<int> edge_local;
   for (int t = 0; t < T.ntiles; ++t) {
     tiles[t].edge_off = static_cast<int>(edge_local.size());
-    for (const auto &gl : T.tile_glob_local[t]) {
-      const uint8_t m = fmask[T.glob2dev[gl.first]];
-      if (m) edge_local.push_back(gl.second | (static_cast<int>(m) << 16));
+    for (int l = 0; l < tiles[t].n_int + tiles[t].n_sh; ++l) {
+      const uint8_t m = fmask[T.glob2dev[T.glob_of(t, l)]];
+      if (m) edge_local.push_back(l | (static_cast<int>(m) << 16));
     }
     tiles[t].edge_n = static_cast<int>(edge_local.size()) - tiles[t].edge_off;
   }
@@ -550,7 +577,6 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   err = build_boundary_groups(tiles, st_local, cpl_local, src_local, bgroups, bnd_idx);
   if (!err.empty()) return fail(SF2D_ERR_INVALID, err);
 
-  AcParams &A = C->A;
   C->nglob = ad->nglob;
   float *p, *pd, *pdd;
   if ((rc = C->alloc(&p, ad->nglob)) || (rc = C->alloc(&pd, ad->nglob)) || (rc = C->alloc(&pdd, ad->nglob))) return rc;
@@ -573,11 +599,11 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
     }
   }
   if ((rc = C->upload_const(&A.rmass, rmass)) || (rc = C->upload_const(&A.free_mask, fmask)) ||
-      (rc = C->upload_const(&A.tiles, tiles)) || (rc = C->upload_const(&A.lib, T.lib)) ||
+      (rc = C->upload_const(&A.tiles, tiles)) || (rc = C->upload_const(&A.lgeo, lgeo)) || (rc = C->upload_const(&A.lfac, lfac)) ||
+      (rc = C->upload_const(&A.lid, lid)) || (rc = C->upload_const(&A.lphase, lphase)) ||
       (rc = C->upload_const(&A.bgroups, bgroups)) || (rc = C->upload_const(&A.bnd_idx, bnd_idx)) ||
-      (rc = C->upload_const(&A.geo, geo)) || (rc = C->upload_const(&A.fac, fac)) ||
       (rc = C->upload_const(&A.sh_ids, T.sh_ids)) || (rc = C->upload_const(&A.shp_off, T.shp_off)) ||
-      (rc = C->upload_const(&A.slot_pos, slot_pos)) || (rc = C->upload_const(&A.st_local, st_local)) ||
+      (rc = C->upload_const(&A.sh_slot, T.sh_slot)) || (rc = C->upload_const(&A.st_local, st_local)) ||
       (rc = C->upload_const(&A.edge_local, edge_local)) ||
       (rc = C->upload_const(&A.st_wr, st_wr)) || (rc = C->upload_const(&A.cpl_local, cpl_local)) ||
       (rc = C->upload_const(&A.cpl_src, cpl_src)) || (rc = C->upload_const(&A.cpl_nw, cpl_nw)) ||
@@ -591,6 +617,9 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
     A.cpl_pml_u = reinterpret_cast<const float2 *>(C->cpl_fluid.out);
   }
   if (pml_ac) {
+    if ((rc = C->upload_const(&A.lib, T.lib)) || (rc = C->upload_const(&A.geo, geo)) ||
+        (rc = C->upload_const(&A.fac, fac)))
+      return rc;
     if ((rc = C->upload_const(&A.pml_sets, pml_sets)) || (rc = C->upload_const(&A.pml_set_idx, pml_set_idx)) ||
         (rc = C->upload_const(&A.pml_jk, pml_jk)))
       return rc;
@@ -622,11 +651,10 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   if ((rc = C->alloc(&C->seis, nseis))) return rc;
   SF2D_CUDA(cudaMemset(C->seis, 0, sizeof(double) * std::max<size_t>(1, nseis)));
   A.seis = C->seis;
-  // step, step shadow, status, -, chi frame base, kernel frame base
+  // step, -, status, -, chi frame base, kernel frame base
   if ((rc = C->alloc(&C->ctr, 8))) return rc;
   SF2D_CUDA(cudaMemset(C->ctr, 0, 8 * sizeof(int)));
   A.d_step = C->ctr;
-  A.d_step_b = C->ctr + 1;
   A.d_status = C->ctr + 2;
   A.pframe_base = C->ctr + 4;
   A.kp_base = C->ctr + 5;
@@ -650,8 +678,16 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   A.dt2o2 = eld->deltatsquareover2;
   A.shared_begin = T.shared_begin;
   A.nshared = T.nshared;
-  A.max_q = T.max_elems * NGLL2;
-  A.max_local = T.max_local;
+  A.nlane_q = nlane_q;
+  for (int t = C->pml_tile0; t < T.ntiles; ++t) {
+    A.max_q = std::max(A.max_q, T.tiles[t].nelem * NGLL2);
+    A.max_local = std::max(A.max_local, T.tiles[t].n_int + T.tiles[t].n_sh);
+  }
+  for (int m = 0; m < 5; ++m) {
+    double sum = 0.0;
+    for (int k = 0; k < 5; ++k) sum += eld->hprime[5 * m + k];
+    A.hsum[m] = static_cast<float>(sum);
+  }
   for (int k = 0; k < 25; ++k) {
     A.hconst[k] = eld->hprime[k];
     A.hconst[25 + k] = eld->hprimewgll[k];
@@ -662,12 +698,13 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   }
   if ((rc = C->upload(&C->d_dev2glob, T.dev2glob.data(), T.dev2glob.size()))) return rc;
   if ((rc = C->alloc(&C->d_stage, ad->nglob))) return rc;
-  C->smem = ac_smem_layout(A.max_q, A.max_local).total;
+  C->smem = ac_row_smem_layout(A.max_local_l, A.max_elems_l, adjoint).total;
   if (C->smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "fluid tile too large for shared memory");
-  C->tile_fn = pick_ac_tile<false>(C->nt, C->lddrk);
+  C->tile_fn = adjoint ? k_acoustic_rows<false, true>
+                       : C->lddrk ? k_acoustic_rows<true, false> : k_acoustic_rows<false, false>;
   if (pml_ac) {
-    C->pml_fn = pick_ac_tile<true>(C->nt, C->lddrk);
-    C->pml_smem = ac_smem_layout(A.max_q, A.max_local, true).total;
+    C->pml_fn = pick_ac_pml_tile(C->nt, C->lddrk);
+    C->pml_smem = ac_smem_layout(A.max_q, A.max_local).total;
     if (C->pml_smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "fluid tile too large for shared memory");
     if (C->pml_tile0 > 0 && C->pml_tile0 < T.ntiles) {
       SF2D_CUDA(cudaStreamCreateWithPriority(&C->side, cudaStreamNonBlocking, C->el ? C->el->priority : 0));
@@ -1008,19 +1045,18 @@ extern "C" int sf2d_coupled_time_kernels(sf2d_coupled *C, int nstep, float *ms) 
   double acc[4] = {0, 0, 0, 0};
   for (int k = 0; k < nstep; ++k)
     for (int st = 0; st < C->nstage; ++st) {
-      const bool rp = k > 0 && st == 0;
       SF2D_CUDA(cudaEventRecord(ev[0], str));
       C->launch_cpl_fluid(st);
-      C->launch_ac_tile(rp, st);
+      C->launch_ac_tile(st, k);
       SF2D_CUDA(cudaEventRecord(ev[1], str));
-      C->launch_ac_shared(st);
+      C->launch_ac_shared(st, k);
       if (st == C->nstage - 1 && C->A.nrec > 0)  // the step's fluid receivers, on the timed stream
-        sf2d::k_acoustic_receivers<<<(C->A.nrec + 127) / 128, 128, 0, str>>>(C->A);
+        sf2d::k_acoustic_receivers<<<(C->A.nrec + 127) / 128, 128, 0, str>>>(C->A, k);
       SF2D_CUDA(cudaEventRecord(ev[2], str));
       C->launch_cpl_solid(st);
-      if (S) S->launch_tile(rp, st);
+      if (S) S->launch_tile(k > 0 && st == 0, st, 0, k);
       SF2D_CUDA(cudaEventRecord(ev[3], str));
-      if (S) S->launch_shared(st);
+      if (S) S->launch_shared(st, k);
       SF2D_CUDA(cudaEventRecord(ev[4], str));
       SF2D_CUDA(cudaEventSynchronize(ev[4]));
       for (int q = 0; q < 4; ++q) {
@@ -1029,8 +1065,9 @@ extern "C" int sf2d_coupled_time_kernels(sf2d_coupled *C, int nstep, float *ms) 
         acc[q] += t;
       }
     }
+  sf2d::k_acoustic_advance<<<1, 1, 0, str>>>(C->A, nstep);
+  if (S) S->launch_advance(nstep);
   SF2D_CUDA(cudaGetLastError());
-  if (S) S->launch_receivers();
   SF2D_CUDA(cudaStreamSynchronize(str));
   C->steps_done += nstep;
   if (S) S->steps_done += nstep;
@@ -1046,7 +1083,7 @@ extern "C" int sf2d_coupled_layout_info(sf2d_coupled *C, long long *info) {
   if (!C || !info) return fail(SF2D_ERR_INVALID, "bad arguments");
   info[0] = C->T.ntiles;
   info[1] = C->T.nshared;
-  info[2] = C->A.max_local;
+  info[2] = C->T.max_local;
   info[3] = static_cast<long long>(C->smem);
   info[4] = C->T.nglob - C->T.nshared;
   info[5] = static_cast<long long>(C->T.sh_ids.size());
@@ -1064,12 +1101,13 @@ extern "C" int sf2d_coupled_launch_count(sf2d_coupled *C, int nstep, long long *
   using namespace sf2d;
   if (!C || !launches || nstep < 0) return fail(SF2D_ERR_INVALID, "bad arguments");
   const sf2d_solver *S = C->el;
-  long long per_stage = (C->cpl_fluid.n > 0) + (C->pml_tile0 > 0) + (C->pml_tile0 < C->T.ntiles) + 1 +
-                        (C->cpl_solid.n > 0);
-  if (S) per_stage += (C->early ? S->tile_launches(S->late_tile0) + (S->late_tile0 > 0) : S->tile_launches(0)) + 1;
+  long long per_stage = (C->cpl_fluid.n > 0) + (C->pml_tile0 > 0) + (C->pml_tile0 < C->T.ntiles) +
+                        (C->A.nshared > 0) + (C->cpl_solid.n > 0);
+  if (S)
+    per_stage += (C->early ? S->tile_launches(S->late_tile0) + (S->late_tile0 > 0) : S->tile_launches(0)) +
+                 (S->P.nshared > 0);
   const long long chunks = nstep / C->chunk + (nstep % C->chunk ? 1 : 0);
-  *launches = per_stage * C->nstage * nstep + (C->A.nrec > 0 ? nstep : 0) + (S && S->nrec > 0 ? chunks : 0) +
-              ((C->A.pframes != nullptr) + (C->A.kl_ac != nullptr)) * static_cast<long long>(nstep);
+  *launches = per_stage * C->nstage * nstep + (C->A.nrec > 0 ? nstep : 0) + (S ? 2 : 1) * chunks;
   return SF2D_OK;
 }
 
@@ -1088,9 +1126,9 @@ extern "C" int sf2d_coupled_destroy(sf2d_coupled *C) {
 // ---------------------------------------------------------------------------
 // Kernel run of a coupled mesh (sf2d_coupled_fwi_*): the solid path's scheme
 // (sf2d_fwi.cu) over both domains.  The forward solver writes solid
-// displacement frames (its tile kernels) and fluid chi frames (k_fluid_frame)
+// displacement frames and fluid chi frames (the tile kernels)
 // while a segment is recomputed; the adjoint solver (adjoint = 1) reads them
-// in its solid tile kernels and in k_fluid_kernels.
+// in its tile kernels.
 
 namespace {
 
@@ -1104,7 +1142,10 @@ int coupled_reset(sf2d_coupled *C) {
   SF2D_CUDA(cudaMemsetAsync(C->A.p, 0, sizeof(float) * n, s));
   SF2D_CUDA(cudaMemsetAsync(C->A.pd, 0, sizeof(float) * n, s));
   SF2D_CUDA(cudaMemsetAsync(C->A.pdd, 0, sizeof(float) * n, s));
-  if (C->A.kl_ac) SF2D_CUDA(cudaMemsetAsync(C->A.kl_ac, 0, sizeof(float2) * C->A.nslot_q, s));
+  if (C->A.kl_ac) {
+    SF2D_CUDA(cudaMemsetAsync(C->A.kl_ac, 0, sizeof(float) * C->A.nlane_q, s));
+    SF2D_CUDA(cudaMemsetAsync(C->A.kap_glob, 0, sizeof(float) * n, s));
+  }
   const size_t nseis = static_cast<size_t>(C->nrec_total) * C->nstep * 2;
   if (nseis) SF2D_CUDA(cudaMemsetAsync(C->seis, 0, sizeof(double) * nseis, s));
   SF2D_CUDA(cudaMemsetAsync(C->ctr, 0, 3 * sizeof(int), s));
@@ -1129,7 +1170,10 @@ struct sf2d_coupled_fwi {
   float2 *sframes = nullptr, *ckpt_s = nullptr;  // solid: K frames; nseg * 3 * ng_s (u, v, a)
   float *pframes = nullptr, *ckpt_f = nullptr;   // fluid: K frames; nseg * 3 * ng_f (chi, chi_dot, chi_dot_dot)
   std::vector<int> ibool_s, el_rec, ac_rec;      // solid ibool; run receiver index of each solid / fluid receiver
-  std::vector<float> rho_s, kappa_s, mu_s;
+  sf2d::KernelScale scale;
+  int *f_lane = nullptr, *f_point = nullptr;      // fluid kernels to element order (k_fluid_kernels)
+  float2 *f_rk = nullptr;
+  float *f_out = nullptr;
   std::vector<void *> allocs;
   cudaEvent_t ev_fwd = nullptr, ev_adj = nullptr;
   ~sf2d_coupled_fwi() {
@@ -1224,9 +1268,9 @@ extern "C" int sf2d_coupled_fwi_create(const sf2d_elastic_desc *eld, const sf2d_
     F->nspec_s = eld->nspec;
     const size_t nl = static_cast<size_t>(eld->nspec) * 25;
     F->ibool_s.assign(eld->ibool, eld->ibool + nl);
-    F->rho_s.assign(solid_rhostore, solid_rhostore + nl);
-    F->kappa_s.assign(solid_kappastore, solid_kappastore + nl);
-    F->mu_s.assign(eld->mustore, eld->mustore + nl);
+    auto dev_alloc = [&](void **q, size_t bytes) { return F->alloc(reinterpret_cast<unsigned char **>(q), bytes); };
+    if (int rc = F->scale.prepare(aj->el, eld->nspec, eld->ibool, solid_rhostore, solid_kappastore, eld->mustore, dev_alloc))
+      return rc;
     F->el_rec.assign(cp->el_rec_global, cp->el_rec_global + eld->nrec);
   }
   int rc = 0;
@@ -1236,24 +1280,24 @@ extern "C" int sf2d_coupled_fwi_create(const sf2d_elastic_desc *eld, const sf2d_
   if (solid && ((rc = F->alloc(&F->sframes, K * F->ng_s)) ||
                 (rc = F->alloc(&F->ckpt_s, static_cast<size_t>(F->nseg) * 3 * F->ng_s))))
     return rc;
-  // fluid kernel accumulation: per element point (slot order) its point, rho, kappa
+  // fluid kernel sums, and what brings them to element order
   {
     const Tiling &T = aj->T;
     const size_t nq = static_cast<size_t>(ad->nspec) * 25;
-    std::vector<int> sib(nq);
+    std::vector<int> row(ad->nspec), pt(nq);
     std::vector<float2> rk(nq);
-    for (int sl = 0; sl < ad->nspec; ++sl)
-      for (int q = 0; q < 25; ++q) {
-        const size_t p = static_cast<size_t>(T.elem_order[sl]) * 25 + q;
-        sib[static_cast<size_t>(sl) * 25 + q] = T.glob2dev[ad->ibool[p]];
-        rk[static_cast<size_t>(sl) * 25 + q] = make_float2(ad->rhostore[p], ad->kappastore[p]);
-      }
+    for (int sl = 0; sl < ad->nspec; ++sl) row[T.elem_order[sl]] = aj->slot_lane[sl];
+    for (size_t p = 0; p < nq; ++p) {
+      pt[p] = T.glob2dev[ad->ibool[p]];
+      rk[p] = make_float2(ad->rhostore[p], ad->kappastore[p]);
+    }
     AcParams &A = aj->A;
-    if ((rc = aj->upload_const(&A.slot_ibool, sib)) || (rc = aj->upload_const(&A.slot_rk, rk)) ||
-        (rc = aj->alloc(&A.kl_ac, nq)))
+    if ((rc = aj->upload(&F->f_lane, row.data(), row.size())) || (rc = aj->upload(&F->f_point, pt.data(), pt.size())) ||
+        (rc = aj->upload(&F->f_rk, rk.data(), rk.size())) || (rc = aj->alloc(&F->f_out, 2 * nq)) ||
+        (rc = aj->alloc(&A.kl_ac, A.nlane_q)) || (rc = aj->alloc(&A.kap_glob, ad->nglob)))
       return rc;
-    SF2D_CUDA(cudaMemset(A.kl_ac, 0, sizeof(float2) * std::max<size_t>(nq, 1)));
-    A.nslot_q = static_cast<int>(nq);
+    SF2D_CUDA(cudaMemset(A.kl_ac, 0, sizeof(float) * std::max<size_t>(A.nlane_q, 1)));
+    SF2D_CUDA(cudaMemset(A.kap_glob, 0, sizeof(float) * ad->nglob));
     A.kpframes = F->pframes;
     A.npframes = F->K;
     // the forward solver's fluid tiling is the adjoint one's (same mesh, same options)
@@ -1369,39 +1413,17 @@ extern "C" int sf2d_coupled_fwi_backward(sf2d_coupled_fwi *F, const float *adj_s
   if (st && st != SF2D_ERR_UNSTABLE) return st;
   if ((rc = put_ctr(C->ctr, 4, NO_FRAMES, sf))) return rc;
   if (solid && (rc = put_ctr(C->el->ctr, 3, NO_FRAMES, sf))) return rc;
-  // solid kernel sums back to the sub-mesh layout with save_kernels_elastic's scaling
-  if (solid) {
-    const sf2d_solver *S = A->el;
-    std::vector<float2> kmu(S->nq);
-    std::vector<float> rg(ns);
-    SF2D_CUDA(cudaMemcpy(kmu.data(), S->P.kmu_kl, sizeof(float2) * S->nq, cudaMemcpyDeviceToHost));
-    SF2D_CUDA(cudaMemcpy(rg.data(), S->P.rho_kl_glob, sizeof(float) * ns, cudaMemcpyDeviceToHost));
-    const sf2d::Tiling &T = S->T;
-    const float dt = F->dt;
-    for (int sl = 0; sl < F->nspec_s; ++sl) {
-      const int e = T.elem_order[sl];
-      for (int q = 0; q < 25; ++q) {
-        const size_t p = static_cast<size_t>(e) * 25 + q;
-        const float rsum = rg[T.glob2dev[F->ibool_s[p]]];
-        const float2 km = kmu[static_cast<size_t>(sl) * 25 + q];
-        rho_kl[p] = -F->rho_s[p] * dt * rsum;
-        mu_kl[p] = -2.f * F->mu_s[p] * dt * km.y;
-        kappa_kl[p] = -F->kappa_s[p] * dt * km.x;
-      }
-    }
-  }
-  // fluid sums (deltat and 1/rho, 1/kappa already in) back to element order
+  // solid kernel sums to the sub-mesh layout with save_kernels_elastic's scaling
+  if (solid && (rc = F->scale.fetch(A->el, F->dt, rho_kl, kappa_kl, mu_kl))) return rc;
+  // fluid sums to element order, with 1/rho, 1/kappa and deltat
   {
-    std::vector<float2> kl(A->A.nslot_q);
-    SF2D_CUDA(cudaMemcpy(kl.data(), A->A.kl_ac, sizeof(float2) * kl.size(), cudaMemcpyDeviceToHost));
-    const sf2d::Tiling &T = A->T;
-    for (int sl = 0; sl < F->nspec_f; ++sl) {
-      const size_t e = static_cast<size_t>(T.elem_order[sl]);
-      for (int q = 0; q < 25; ++q) {
-        rho_ac_kl[e * 25 + q] = kl[static_cast<size_t>(sl) * 25 + q].x;
-        kappa_ac_kl[e * 25 + q] = kl[static_cast<size_t>(sl) * 25 + q].y;
-      }
-    }
+    const int n = F->nspec_f * NGLL2;
+    k_fluid_kernels<<<(n + 255) / 256, 256, 0, sa>>>(A->A.kl_ac, A->A.kap_glob, F->f_lane, F->f_point, F->f_rk, F->dt, n,
+                                                      F->f_out);
+    SF2D_CUDA(cudaGetLastError());
+    SF2D_CUDA(cudaMemcpyAsync(rho_ac_kl, F->f_out, sizeof(float) * n, cudaMemcpyDeviceToHost, sa));
+    SF2D_CUDA(cudaMemcpyAsync(kappa_ac_kl, F->f_out + n, sizeof(float) * n, cudaMemcpyDeviceToHost, sa));
+    SF2D_CUDA(cudaStreamSynchronize(sa));
   }
   return st;
 }
@@ -1430,7 +1452,7 @@ extern "C" int sf2d_coupled_fwi_kernel_sums(sf2d_coupled_fwi *F, float *rho_kl, 
     const int e = T.elem_order[sl];
     for (int q = 0; q < 25; ++q) {
       const size_t p = static_cast<size_t>(e) * 25 + q;
-      const float2 km = kmu[static_cast<size_t>(sl) * 25 + q];
+      const float2 km = kmu[S->lane_index(sl, q)];
       rho_kl[p] = rg[T.glob2dev[F->ibool_s[p]]];
       kappa_kl[p] = km.x;
       mu_kl[p] = km.y;

@@ -3,10 +3,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -15,6 +17,7 @@
 
 #include "sf2d_b200.h"
 #include "sf2d_kernels.cuh"
+#include "sf2d_rows.cuh"
 #include "sf2d_tiler.h"
 
 #include "sf2d_runtime.h"
@@ -105,10 +108,13 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
 
   auto *S = new sf2d_solver();
   std::unique_ptr<sf2d_solver> guard(S);
-  const int te = d->tile_elems > 0 ? d->tile_elems : 64;
-  const int group_te[3] = {te, te, d->pml_tile_elems > 0 ? d->pml_tile_elems : te};
+  if (d->tile_elems > 256) return fail(SF2D_ERR_INVALID, "tiling: tile_elems must be in [1, 256]");
+  // five threads an element and at most 96 registers a thread: 128 elements fit the register file
+  const int te = std::min(d->tile_elems > 0 ? d->tile_elems : 64, 128);
+  const int group_te[3] = {te, te, d->pml_tile_elems > 0 ? d->pml_tile_elems : d->tile_elems > 0 ? d->tile_elems : 64};
   std::string err = build_tiling(d->nspec, d->nglob, d->ibool, d->centroid_xz, te, S->T,
-                                 grouped ? group.data() : nullptr, grouped ? 3 : 1, grouped ? group_te : nullptr);
+                                 grouped ? group.data() : nullptr, grouped ? 3 : 1, grouped ? group_te : nullptr,
+                                 grouped ? 2 : 1);
   if (!err.empty()) return fail(SF2D_ERR_INVALID, "tiling: " + err);
   const Tiling &T = S->T;
   S->late_tile0 = late_elem ? T.group_tile_begin[1] : 0;
@@ -119,48 +125,97 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   for (int k = 0; k < d->nstacey; ++k)
     if (d->st_iglob[k] < 0 || d->st_iglob[k] >= d->nglob) return fail(SF2D_ERR_INVALID, "Stacey point out of range");
 
-  // per-slot element data
-  const size_t nq = static_cast<size_t>(d->nspec) * NGLL2;
-  std::vector<float4> geo(nq);
-  std::vector<float2> mat(nq);
-  for (int s = 0; s < d->nspec; ++s) {
-    const size_t src = static_cast<size_t>(T.elem_order[s]) * NGLL2;
-    for (int q = 0; q < NGLL2; ++q) {
-      geo[s * NGLL2 + q] = make_float4(d->xix[src + q], d->xiz[src + q], d->gammax[src + q], d->gammaz[src + q]);
-      mat[s * NGLL2 + q] = make_float2(d->lambdastore[src + q], d->mustore[src + q]);
-    }
-  }
-  // anisotropic blocks, in slot order
-  std::vector<int> aniso_idx;
-  std::vector<float4> c4;
-  std::vector<float2> c2;
-  if (aniso) {
-    aniso_idx.assign(d->nspec, -1);
-    int na = 0;
-    for (int s = 0; s < d->nspec; ++s) {
-      const int e = T.elem_order[s];
-      if (!d->ispec_is_anisotropic[e]) continue;
-      aniso_idx[s] = na++;
+  // element data of the tiles by rows (sf2d_rows.cuh)
+  S->pml_tile0 = grouped ? T.group_tile_begin[2] : T.ntiles;
+  const int pml_slot0 = S->pml_tile0 < T.ntiles ? T.tiles[S->pml_tile0].elem_base : d->nspec;
+  S->slot_lane.resize(pml_slot0);
+  for (int t = 0; t < S->pml_tile0; ++t)
+    for (int k = 0; k < T.tiles[t].nelem; ++k) S->slot_lane[T.tiles[t].elem_base + k] = T.tiles[t].lane0 + 5 * k;
+  const size_t nq = static_cast<size_t>(T.nlanes) * 5;  // element points, tiles padded to whole warps
+  std::vector<float4> lgeo(nq, make_float4(0.f, 0.f, 0.f, 0.f));
+  std::vector<float2> lmat(nq, make_float2(0.f, 0.f));
+  std::vector<uint32_t> rid(static_cast<size_t>(T.nlanes) * 3, 0);
+  std::vector<uint32_t> lphase(T.phases.begin(), T.phases.begin() + pml_slot0);
+  std::vector<int> lani;
+  std::vector<float4> lc4;
+  std::vector<float2> lc2;
+  if (aniso) lani.assign(pml_slot0, -1);
+  for (int t = 0; t < S->pml_tile0; ++t) {
+    const TileInfo &ti = T.tiles[t];
+    for (int k = 0; k < ti.nelem; ++k) {
+      const int s = ti.elem_base + k, e = T.elem_order[s], r0 = S->slot_lane[s];
       const size_t src = static_cast<size_t>(e) * NGLL2;
+      const uint16_t *lib = &T.lib[static_cast<size_t>(ti.lib_off) + static_cast<size_t>(k) * NGLL2];
       for (int q = 0; q < NGLL2; ++q) {
-        c4.push_back(make_float4(d->c11[src + q], d->c13[src + q], d->c15[src + q], d->c33[src + q]));
-        c2.push_back(make_float2(d->c35[src + q], d->c55[src + q]));
+        const size_t p = src + q;
+        const size_t dst = S->lane_index(s, q);
+        lgeo[dst] = make_float4(d->xix[p], d->xiz[p], d->gammax[p], d->gammaz[p]);
+        lmat[dst] = make_float2(d->lambdastore[p], d->mustore[p]);
+      }
+      for (int j = 0; j < NGLL; ++j) {
+        const int r = r0 + j;
+        const size_t o = static_cast<size_t>(r / 32) * 96 + r % 32;
+        const uint16_t *l = lib + NGLL * j;
+        rid[o] = l[0] | static_cast<uint32_t>(l[1]) << 16;
+        rid[o + 32] = l[2] | static_cast<uint32_t>(l[3]) << 16;
+        rid[o + 64] = l[4] | static_cast<uint32_t>(lib[12]) << 16;
+      }
+      if (aniso && d->ispec_is_anisotropic[e]) {
+        lphase[s] |= 0x80000000u;
+        lani[s] = static_cast<int>(lc4.size() / NGLL2);
+        for (int q = 0; q < NGLL2; ++q) {
+          const size_t p = src + q;
+          lc4.push_back(make_float4(d->c11[p], d->c13[p], d->c15[p], d->c33[p]));
+          lc2.push_back(make_float2(d->c35[p], d->c55[p]));
+        }
       }
     }
   }
-  // attenuation coefficients: 3 float4 per element point, slot order
-  std::vector<float4> att_coef;
+  // CPML tiles: per slot
+  std::vector<float4> geo;
+  std::vector<float2> mat;
+  for (int s = pml_slot0; s < d->nspec; ++s)
+    for (int q = 0; q < NGLL2; ++q) {
+      const size_t p = static_cast<size_t>(T.elem_order[s]) * NGLL2 + q;
+      geo.push_back(make_float4(d->xix[p], d->xiz[p], d->gammax[p], d->gammaz[p]));
+      mat.push_back(make_float2(d->lambdastore[p], d->mustore[p]));
+    }
+  // attenuation coefficients: sets of equal values, named per element or, when
+  // some element mixes them, per point
+  std::vector<float4> att_sets;
+  std::vector<int> att_eset, att_pset;
   if (atten) {
-    att_coef.resize(nq * 3);
     const float *k0 = lddrk ? d->att_itau1 : d->att_a1, *k1 = lddrk ? d->att_itau2 : d->att_a2;
     const float *k2 = lddrk ? d->att_phi1 : d->att_b1, *k3 = lddrk ? d->att_phi2 : d->att_b2;
-    for (int s = 0; s < d->nspec; ++s) {
-      const size_t src = static_cast<size_t>(T.elem_order[s]) * NGLL2;
-      for (int q = 0; q < NGLL2; ++q)
-        for (int l = 0; l < 3; ++l) {
-          const size_t o = (src + q) * 3 + l;
-          att_coef[(static_cast<size_t>(s) * NGLL2 + q) * 3 + l] = make_float4(k0[o], k1[o], k2[o], k3[o]);
+    std::map<std::array<uint32_t, 12>, int> seen;
+    std::vector<int> pset(nq, 0);
+    std::array<uint32_t, 12> key{}, prev{};
+    int id = -1;
+    bool mixed = false;
+    for (int s = 0; s < pml_slot0; ++s)
+      for (int q = 0; q < NGLL2; ++q) {
+        const size_t p = (static_cast<size_t>(T.elem_order[s]) * NGLL2 + q) * 3;
+        std::memcpy(&key[0], k0 + p, 12);
+        std::memcpy(&key[3], k1 + p, 12);
+        std::memcpy(&key[6], k2 + p, 12);
+        std::memcpy(&key[9], k3 + p, 12);
+        if (id < 0 || key != prev) {
+          const auto it = seen.emplace(key, static_cast<int>(seen.size()));
+          id = it.first->second;
+          if (it.second) {
+            for (int l = 0; l < 3; ++l) att_sets.push_back(make_float4(k0[p + l], k1[p + l], k2[p + l], k3[p + l]));
+          }
+          prev = key;
         }
+        pset[S->lane_index(s, q)] = id;
+        if (q > 0 && pset[S->lane_index(s, 0)] != id) mixed = true;
+      }
+    if (att_sets.empty()) att_sets.assign(4, make_float4(0.f, 0.f, 0.f, 0.f));
+    if (mixed) {
+      att_pset.swap(pset);
+    } else {
+      att_eset.resize(pml_slot0);
+      for (int s = 0; s < pml_slot0; ++s) att_eset[s] = pset[S->lane_index(s, 0)];
     }
   }
   std::vector<float2> rmass(d->nglob);
@@ -215,8 +270,6 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   }
   // CPML layer: element slots [pml_slot0, nspec) (the last tiles), per-point
   // damping data, the outer edge as per-tile local lists and a shared-point mask
-  S->pml_tile0 = grouped ? T.group_tile_begin[2] : T.ntiles;
-  const int pml_slot0 = S->pml_tile0 < T.ntiles ? T.tiles[S->pml_tile0].elem_base : d->nspec;
   std::vector<int> pml_set_idx, edge_local, pml_vset_idx;
   std::vector<PmlSet> pml_sets;
   std::vector<PmlVisco> pml_vsets;
@@ -235,8 +288,8 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     for (int k = 0; k < d->npml_edge; ++k) on_edge[d->pml_edge_iglob[k]] = 1;
     for (int t = 0; t < T.ntiles; ++t) {
       tiles[t].edge_off = static_cast<int>(edge_local.size());
-      for (const auto &gl : T.tile_glob_local[t])
-        if (on_edge[gl.first]) edge_local.push_back(gl.second);
+      for (int l = 0; l < tiles[t].n_int + tiles[t].n_sh; ++l)
+        if (on_edge[T.glob_of(t, l)]) edge_local.push_back(l);
       tiles[t].edge_n = static_cast<int>(edge_local.size()) - tiles[t].edge_off;
     }
     sh_edge.assign(std::max(T.nshared, 1), 0);
@@ -277,16 +330,13 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   } while (0)
   UP(rmass, float2, rmass);
   UP(tiles, TileInfo, tiles);
-  UP(lib, uint16_t, T.lib);
-  UP(geo, float4, geo);
-  UP(mat, float2, mat);
+  UP(rgeo, float4, lgeo);
+  UP(rmat, float2, lmat);
+  UP(rid, uint32_t, rid);
+  UP(rphase, uint32_t, lphase);
   UP(sh_ids, int, T.sh_ids);
   UP(shp_off, int, T.shp_off);
-  {
-    std::vector<int> slot_pos(T.shp_slots.size());
-    for (size_t k = 0; k < T.shp_slots.size(); ++k) slot_pos[T.shp_slots[k]] = static_cast<int>(k);
-    UP(slot_pos, int, slot_pos);
-  }
+  UP(sh_slot, int, T.sh_slot);
   UP(bgroups, int4, bgroups);
   UP(bnd_idx, int, bnd_idx);
   UP(st_local, int, st_local);
@@ -299,21 +349,22 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   UP(rec_dev, int, rec_dev);
   UP(rec_h, double, rec_h);
   if (aniso) {
-    UP(aniso_idx, int, aniso_idx);
-    UP(c4, float4, c4);
-    UP(c2, float2, c2);
+    UP(rani, int, lani);
+    UP(rc4, float4, lc4);
+    UP(rc2, float2, lc2);
   }
   if (atten) {
-    UP(att_coef, float4, att_coef);
-    float4 *st = nullptr;
-    if ((rc = S->alloc(&st, nq * 3))) return rc;
-    SF2D_CUDA(cudaMemset(st, 0, sizeof(float4) * nq * 3));
-    P.att_state = st;
+    UP(att_sets, float4, att_sets);
+    if (!att_eset.empty()) UP(att_eset, int, att_eset);
+    if (!att_pset.empty()) UP(att_pset, int, att_pset);
+    S->att_bytes = lddrk ? (sizeof(float4) * 4 + sizeof(float) * 2) * nq : sizeof(float4) * 3 * nq;
+    if ((rc = S->alloc(&S->att_buf, S->att_bytes))) return rc;
+    SF2D_CUDA(cudaMemset(S->att_buf, 0, S->att_bytes));
+    P.att_a = reinterpret_cast<float4 *>(S->att_buf);
     if (lddrk) {
-      float4 *stl = nullptr;
-      if ((rc = S->alloc(&stl, nq * 3))) return rc;
-      SF2D_CUDA(cudaMemset(stl, 0, sizeof(float4) * nq * 3));
-      P.att_state_l = stl;
+      P.att_al = P.att_a + 2 * nq;
+      P.att_c = reinterpret_cast<float *>(P.att_al + 2 * nq);
+      P.att_cl = P.att_c + nq;
     }
   }
   if (lddrk) {
@@ -329,6 +380,9 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     }
   }
   if (pml) {
+    UP(lib, uint16_t, T.lib);
+    UP(geo, float4, geo);
+    UP(mat, float2, mat);
     UP(pml_sets, PmlSet, pml_sets);
     UP(pml_set_idx, int, pml_set_idx);
     UP(pml_rhoj, float, pml_rhoj);
@@ -375,7 +429,6 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   SF2D_CUDA(cudaMemset(ctr, 0, 8 * sizeof(int)));
   P.d_step = ctr;
   P.d_status = ctr + 1;
-  P.d_step_b = ctr + 2;
   P.frame_base = ctr + 3;
   P.kern_base = ctr + 4;
   P.nglob = d->nglob;
@@ -408,8 +461,11 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   P.dt2o2 = d->deltatsquareover2;
   P.shared_begin = T.shared_begin;
   P.nshared = T.nshared;
-  P.max_q = T.max_elems * NGLL2;
-  P.max_local = T.max_local;
+  for (int t = 0; t < S->pml_tile0; ++t) {
+    P.max_elems = std::max(P.max_elems, tiles[t].nelem);
+    S->lane_nt = std::max(S->lane_nt, (5 * tiles[t].nelem + 31) / 32 * 32);
+    P.max_local = std::max(P.max_local, tiles[t].n_int + tiles[t].n_sh);
+  }
   for (int k = 0; k < 25; ++k) {
     P.hconst[k] = d->hprime[k];
     P.hconst[25 + k] = d->hprimewgll[k];
@@ -418,7 +474,7 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     P.hconst[50 + k] = d->wxgll[k];
     P.hconst[55 + k] = d->wzgll[k];
   }
-  S->smem = tile_smem_layout(P.max_q, P.max_local, kern).total;
+  S->smem = row_smem_layout(P.max_local, P.max_elems, kern).total;
   if (S->smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "tile too large for shared memory");
   S->nt = d->threads_per_block > 0 ? d->threads_per_block : 256;
   if (S->nt != 128 && S->nt != 250 && S->nt != 256 && S->nt != 512)
@@ -427,11 +483,16 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   if (S->pml_nt != 128 && S->pml_nt != 250 && S->pml_nt != 256 && S->pml_nt != 512)
     return fail(SF2D_ERR_INVALID, "pml_threads_per_block must be 128, 250, 256 or 512");
   if (d->nrec > 0) {
-    for (int t = 0; t < T.ntiles; ++t)
-      if (tiles[t].rec_n > (t < S->pml_tile0 ? S->nt : S->pml_nt))
+    for (int t = S->pml_tile0; t < T.ntiles; ++t)
+      if (tiles[t].rec_n > S->pml_nt)
         return fail(SF2D_ERR_INVALID, "more receivers in one tile than threads per CTA");
   }
-  S->tile_fn = pick_tile_kernel(S->nt, aniso, atten, lddrk, kern);
+  for (int m = 0; m < 5; ++m) {
+    double sum = 0.0;
+    for (int k = 0; k < 5; ++k) sum += d->hprime[5 * m + k];
+    P.hsum[m] = static_cast<float>(sum);
+  }
+  S->tile_fn = pick_rows_kernel(aniso, atten, lddrk, kern);
   if (pml) {
     // the layer's tiles may be smaller than the others: their kernel gets its
     // own shared-memory layout (the largest layer tile's)
@@ -443,7 +504,7 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     S->pml_max_q = pe * NGLL2;
     S->pml_max_local = pl;
     S->pml_fn = pick_pml_kernel(S->pml_nt, lddrk, pml_visco);
-    S->pml_smem = tile_smem_layout(S->pml_max_q, S->pml_max_local, false, true).total;
+    S->pml_smem = tile_smem_layout(S->pml_max_q, S->pml_max_local).total;
     if (S->pml_smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "tile too large for shared memory");
   }
   S->lddrk = lddrk;
@@ -565,7 +626,8 @@ extern "C" int sf2d_synchronize(sf2d_solver *S, double timeout_s) {
   if (!S) return fail(SF2D_ERR_INVALID, "null solver");
   const auto t0 = std::chrono::steady_clock::now();
   for (;;) {
-    cudaError_t e = cudaStreamQuery(S->stream);
+    // without a limit the driver's own wait returns as the steps end
+    cudaError_t e = timeout_s > 0 ? cudaStreamQuery(S->stream) : cudaStreamSynchronize(S->stream);
     if (e == cudaSuccess) break;
     if (e != cudaErrorNotReady) return fail(SF2D_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
     if (timeout_s > 0 &&
@@ -693,12 +755,12 @@ extern "C" int sf2d_time_kernels(sf2d_solver *S, int nstep, float *ms) {
     for (int st = 0; st < ns; ++st) {
       const size_t b = (static_cast<size_t>(k) * ns + st) * 3;
       SF2D_CUDA(cudaEventRecord(ev[b], S->stream));
-      S->launch_tile(k > 0 && st == 0, st);
+      S->launch_tile(k > 0 && st == 0, st, 0, k);
       SF2D_CUDA(cudaEventRecord(ev[b + 1], S->stream));
-      S->launch_shared(st);
+      S->launch_shared(st, k);
       SF2D_CUDA(cudaEventRecord(ev[b + 2], S->stream));
     }
-  S->launch_receivers();
+  S->launch_advance(nstep);
   SF2D_CUDA(cudaGetLastError());
   SF2D_CUDA(cudaStreamSynchronize(S->stream));
   double a = 0, bsum = 0;
@@ -726,16 +788,16 @@ extern "C" int sf2d_layout_info(sf2d_solver *S, long long *info) {
   info[3] = S->T.max_elems;
   info[4] = static_cast<long long>(S->dev_bytes);
   info[5] = static_cast<long long>(S->smem);
-  info[6] = S->nt;
+  info[6] = S->lane_nt;
   info[7] = static_cast<long long>(S->T.sh_ids.size());
   return SF2D_OK;
 }
 
 extern "C" int sf2d_launch_count(sf2d_solver *S, int nstep, long long *launches) {
   if (!S || !launches || nstep < 0) return fail(SF2D_ERR_INVALID, "bad arguments");
-  const long long per_stage = S->tile_launches(0) + 1;
+  const long long per_stage = S->tile_launches(0) + (S->P.nshared > 0);
   const long long chunks = nstep / S->chunk + (nstep % S->chunk ? 1 : 0);
-  *launches = per_stage * S->nstage * nstep + (S->nrec > 0 ? chunks : 0);
+  *launches = per_stage * S->nstage * nstep + chunks;
   return SF2D_OK;
 }
 
@@ -754,8 +816,7 @@ int sf2d_reset_solver(sf2d_solver *S) {
   SF2D_CUDA(cudaMemsetAsync(P.a, 0, sizeof(float2) * ng, S->stream));
   if (P.uL) SF2D_CUDA(cudaMemsetAsync(P.uL, 0, sizeof(float2) * ng, S->stream));
   if (P.vL) SF2D_CUDA(cudaMemsetAsync(P.vL, 0, sizeof(float2) * ng, S->stream));
-  if (P.att_state) SF2D_CUDA(cudaMemsetAsync(P.att_state, 0, sizeof(float4) * S->nq * 3, S->stream));
-  if (P.att_state_l) SF2D_CUDA(cudaMemsetAsync(P.att_state_l, 0, sizeof(float4) * S->nq * 3, S->stream));
+  if (S->att_buf) SF2D_CUDA(cudaMemsetAsync(S->att_buf, 0, S->att_bytes, S->stream));
   if (P.kmu_kl) SF2D_CUDA(cudaMemsetAsync(P.kmu_kl, 0, sizeof(float2) * S->nq, S->stream));
   if (P.rho_kl_glob) SF2D_CUDA(cudaMemsetAsync(P.rho_kl_glob, 0, sizeof(float) * ng, S->stream));
   if (P.hess_glob) SF2D_CUDA(cudaMemsetAsync(P.hess_glob, 0, sizeof(float2) * ng, S->stream));

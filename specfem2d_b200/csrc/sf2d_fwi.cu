@@ -24,9 +24,9 @@ struct sf2d_fwi {
   float2 *frames = nullptr;
   float2 *aframes = nullptr;  // forward accelerations, with the approximate Hessian
   float2 *ckpt = nullptr;     // nseg * 3 * nglob (u, v, a)
-  float4 *ckpt_att = nullptr; // nseg * 3 * nq (memory variables and old strains)
+  unsigned char *ckpt_att = nullptr; // nseg * att_bytes (memory variables and old strains)
   std::vector<int> ibool;
-  std::vector<float> rho, kappa, mu;
+  sf2d::KernelScale scale;
   std::vector<void *> allocs;
   cudaEvent_t ev_fwd = nullptr, ev_adj = nullptr;
   ~sf2d_fwi() {
@@ -89,9 +89,6 @@ extern "C" int sf2d_fwi_create(const sf2d_elastic_desc *d, const float *rhostore
   F->dt = d->deltat;
   const size_t nl = static_cast<size_t>(d->nspec) * 25;
   F->ibool.assign(d->ibool, d->ibool + nl);
-  F->rho.assign(rhostore, rhostore + nl);
-  F->kappa.assign(kappastore, kappastore + nl);
-  F->mu.assign(d->mustore, d->mustore + nl);
   auto dev_alloc = [&](void **p, size_t bytes) -> int {
     cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
     if (e != cudaSuccess)
@@ -100,11 +97,11 @@ extern "C" int sf2d_fwi_create(const sf2d_elastic_desc *d, const float *rhostore
     F->allocs.push_back(*p);
     return SF2D_OK;
   };
+  if ((rc = F->scale.prepare(F->adj, d->nspec, d->ibool, rhostore, kappastore, d->mustore, dev_alloc))) return rc;
   const size_t ng = static_cast<size_t>(d->nglob);
   if ((rc = dev_alloc(reinterpret_cast<void **>(&F->frames), sizeof(float2) * ng * F->K))) return rc;
   if ((rc = dev_alloc(reinterpret_cast<void **>(&F->ckpt), sizeof(float2) * ng * 3 * F->nseg))) return rc;
-  if (F->fwd->atten &&
-      (rc = dev_alloc(reinterpret_cast<void **>(&F->ckpt_att), sizeof(float4) * F->fwd->nq * 3 * F->nseg)))
+  if (F->fwd->atten && (rc = dev_alloc(reinterpret_cast<void **>(&F->ckpt_att), F->fwd->att_bytes * F->nseg)))
     return rc;
   SF2D_CUDA(cudaEventCreateWithFlags(&F->ev_fwd, cudaEventDisableTiming));
   SF2D_CUDA(cudaEventCreateWithFlags(&F->ev_adj, cudaEventDisableTiming));
@@ -131,8 +128,8 @@ extern "C" int sf2d_fwi_forward(sf2d_fwi *F, double *seismograms) {
     SF2D_CUDA(cudaMemcpyAsync(ck + ng, S->P.v, sizeof(float2) * ng, cudaMemcpyDeviceToDevice, S->stream));
     SF2D_CUDA(cudaMemcpyAsync(ck + 2 * ng, S->P.a, sizeof(float2) * ng, cudaMemcpyDeviceToDevice, S->stream));
     if (F->ckpt_att)
-      SF2D_CUDA(cudaMemcpyAsync(F->ckpt_att + static_cast<size_t>(seg) * 3 * S->nq, S->P.att_state,
-                                sizeof(float4) * 3 * S->nq, cudaMemcpyDeviceToDevice, S->stream));
+      SF2D_CUDA(cudaMemcpyAsync(F->ckpt_att + S->att_bytes * seg, S->att_buf, S->att_bytes, cudaMemcpyDeviceToDevice,
+                                S->stream));
     const int n = std::min(F->K, F->nstep - seg * F->K);
     if ((rc = sf2d_enqueue(S, n))) return rc;
   }
@@ -159,7 +156,6 @@ extern "C" int sf2d_fwi_backward(sf2d_fwi *F, const float *adj_src, float *rho_k
   int rc = sf2d_reset_solver(A);
   if (rc) return rc;
   const size_t ng = static_cast<size_t>(F->nglob);
-  std::vector<int> bases(static_cast<size_t>(2 * F->nseg));
   for (int seg = F->nseg - 1; seg >= 0; --seg) {
     const int s0 = seg * F->K;
     const int n = std::min(F->K, nstep - s0);
@@ -170,8 +166,8 @@ extern "C" int sf2d_fwi_backward(sf2d_fwi *F, const float *adj_src, float *rho_k
     SF2D_CUDA(cudaMemcpyAsync(S->P.v, ck + ng, sizeof(float2) * ng, cudaMemcpyDeviceToDevice, S->stream));
     SF2D_CUDA(cudaMemcpyAsync(S->P.a, ck + 2 * ng, sizeof(float2) * ng, cudaMemcpyDeviceToDevice, S->stream));
     if (F->ckpt_att)
-      SF2D_CUDA(cudaMemcpyAsync(S->P.att_state, F->ckpt_att + static_cast<size_t>(seg) * 3 * S->nq,
-                                sizeof(float4) * 3 * S->nq, cudaMemcpyDeviceToDevice, S->stream));
+      SF2D_CUDA(cudaMemcpyAsync(S->att_buf, F->ckpt_att + S->att_bytes * seg, S->att_bytes, cudaMemcpyDeviceToDevice,
+                                S->stream));
     if ((rc = set_ctr(S, 0, s0)) || (rc = set_ctr(S, 3, s0))) return rc;
     if ((rc = sf2d_enqueue(S, n))) return rc;
     SF2D_CUDA(cudaEventRecord(F->ev_fwd, S->stream));
@@ -185,24 +181,8 @@ extern "C" int sf2d_fwi_backward(sf2d_fwi *F, const float *adj_src, float *rho_k
   const int st = sf2d_synchronize(A, 0.0);
   if (st && st != SF2D_ERR_UNSTABLE) return st;
   if ((rc = set_ctr(S, 3, 1 << 30))) return rc;
-  // kernel sums back to the reference layout, then save_kernels_elastic scaling
-  std::vector<float2> kmu(A->nq);
-  std::vector<float> rg(ng);
-  SF2D_CUDA(cudaMemcpy(kmu.data(), A->P.kmu_kl, sizeof(float2) * A->nq, cudaMemcpyDeviceToHost));
-  SF2D_CUDA(cudaMemcpy(rg.data(), A->P.rho_kl_glob, sizeof(float) * ng, cudaMemcpyDeviceToHost));
-  const sf2d::Tiling &T = A->T;
-  const float dt = F->dt;
-  for (int sl = 0; sl < F->nspec; ++sl) {
-    const int e = T.elem_order[sl];
-    for (int q = 0; q < 25; ++q) {
-      const size_t p = static_cast<size_t>(e) * 25 + q;
-      const float rsum = rg[T.glob2dev[F->ibool[p]]];
-      const float2 km = kmu[static_cast<size_t>(sl) * 25 + q];
-      rho_kl[p] = -F->rho[p] * dt * rsum;
-      mu_kl[p] = -2.f * F->mu[p] * dt * km.y;
-      kappa_kl[p] = -F->kappa[p] * dt * km.x;
-    }
-  }
+  // kernel sums to the reference layout with save_kernels_elastic's scaling
+  if ((rc = F->scale.fetch(A, F->dt, rho_kl, kappa_kl, mu_kl))) return rc;
   return st;
 }
 
@@ -267,7 +247,7 @@ extern "C" int sf2d_fwi_kernel_sums(sf2d_fwi *F, float *rho_kl, float *kappa_kl,
     const int e = T.elem_order[sl];
     for (int q = 0; q < 25; ++q) {
       const size_t p = static_cast<size_t>(e) * 25 + q;
-      const float2 km = kmu[static_cast<size_t>(sl) * 25 + q];
+      const float2 km = kmu[A->lane_index(sl, q)];
       rho_kl[p] = rg[T.glob2dev[F->ibool[p]]];
       kappa_kl[p] = km.x;
       mu_kl[p] = km.y;

@@ -4,11 +4,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <string>
 #include <vector>
 
 #include "sf2d_b200.h"
 #include "sf2d_kernels.cuh"
+#include "sf2d_rows.cuh"
 #include "sf2d_tiler.h"
 
 namespace sf2d {
@@ -29,24 +31,27 @@ using sf2d::fail;
 
 namespace sf2d {
 
-using TileKernel = void (*)(Params, int, int, int);
+using TileKernel = void (*)(Params, int, int, int, int);
 
-template <int NT, bool KERN>
-TileKernel pick_tile_kernel(bool aniso, bool atten, bool lddrk) {
-  if (aniso) {
-    if (atten) return lddrk ? k_elastic_tile<NT, true, true, true, KERN> : k_elastic_tile<NT, true, true, false, KERN>;
-    return lddrk ? k_elastic_tile<NT, true, false, true, KERN> : k_elastic_tile<NT, true, false, false, KERN>;
+inline TileKernel pick_rows_kernel(bool aniso, bool atten, bool lddrk, bool kern) {
+  if (kern) {  // Newmark
+    if (aniso) return atten ? k_elastic_rows<true, true, false, true> : k_elastic_rows<true, false, false, true>;
+    return atten ? k_elastic_rows<false, true, false, true> : k_elastic_rows<false, false, false, true>;
   }
-  if (atten) return lddrk ? k_elastic_tile<NT, false, true, true, KERN> : k_elastic_tile<NT, false, true, false, KERN>;
-  return lddrk ? k_elastic_tile<NT, false, false, true, KERN> : k_elastic_tile<NT, false, false, false, KERN>;
+  if (aniso) {
+    if (atten) return lddrk ? k_elastic_rows<true, true, true, false> : k_elastic_rows<true, true, false, false>;
+    return lddrk ? k_elastic_rows<true, false, true, false> : k_elastic_rows<true, false, false, false>;
+  }
+  if (atten) return lddrk ? k_elastic_rows<false, true, true, false> : k_elastic_rows<false, true, false, false>;
+  return lddrk ? k_elastic_rows<false, false, true, false> : k_elastic_rows<false, false, false, false>;
 }
 
 // the kernel of a CPML layer's tiles (isotropic, forward); visco: some layer
 // elements attenuate (Newmark only)
 template <int NT>
 inline TileKernel pick_pml_kernel(bool lddrk, bool visco) {
-  if (visco) return k_elastic_tile<NT, false, true, false, false, true>;
-  return lddrk ? k_elastic_tile<NT, false, false, true, false, true> : k_elastic_tile<NT, false, false, false, false, true>;
+  if (visco) return k_elastic_pml_tile<NT, true, false>;
+  return lddrk ? k_elastic_pml_tile<NT, false, true> : k_elastic_pml_tile<NT, false, false>;
 }
 inline TileKernel pick_pml_kernel(int nt, bool lddrk, bool visco = false) {
   switch (nt) {
@@ -54,15 +59,6 @@ inline TileKernel pick_pml_kernel(int nt, bool lddrk, bool visco = false) {
     case 250: return pick_pml_kernel<250>(lddrk, visco);
     case 512: return pick_pml_kernel<512>(lddrk, visco);
     default: return pick_pml_kernel<256>(lddrk, visco);
-  }
-}
-
-inline TileKernel pick_tile_kernel(int nt, bool aniso, bool atten, bool lddrk, bool kern) {
-  switch (nt) {
-    case 128: return kern ? pick_tile_kernel<128, true>(aniso, atten, lddrk) : pick_tile_kernel<128, false>(aniso, atten, lddrk);
-    case 250: return kern ? pick_tile_kernel<250, true>(aniso, atten, lddrk) : pick_tile_kernel<250, false>(aniso, atten, lddrk);
-    case 512: return kern ? pick_tile_kernel<512, true>(aniso, atten, lddrk) : pick_tile_kernel<512, false>(aniso, atten, lddrk);
-    default: return kern ? pick_tile_kernel<256, true>(aniso, atten, lddrk) : pick_tile_kernel<256, false>(aniso, atten, lddrk);
   }
 }
 
@@ -129,7 +125,17 @@ struct sf2d_solver {
   int chunk = 32;
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
-  int nt = 256;  // threads per CTA of the tile kernel
+  int nt = 256;      // threads per CTA asked for (the CPML tiles' default)
+  int lane_nt = 32;  // threads per CTA of the tiles by rows: five per element of the largest, in whole warps
+  // tiles by rows: slot -> the element's first row
+  std::vector<int> slot_lane;
+  // index of an element point in the blocks' [q][element] arrays
+  size_t lane_index(int slot, int q) const {
+    const int r = slot_lane[slot] + q / 5;
+    return (static_cast<size_t>(r / 32) * 5 + q % 5) * 32 + r % 32;
+  }
+  unsigned char *att_buf = nullptr;  // every memory variable of the tiles by rows
+  size_t att_bytes = 0;
   int pml_nt = 256, pml_max_q = 0, pml_max_local = 0;  // the CPML tiles' kernel
   int late_tile0 = 0;  // tiles [late_tile0, pml_tile0) touch points another domain uses
   int nmembers = 0;    // members of a packed batch (sf2d_set_members), 0 = none
@@ -153,7 +159,7 @@ struct sf2d_solver {
     if (count) SF2D_CUDA(cudaMemcpy(*p, host, count * sizeof(T_), cudaMemcpyHostToDevice));
     return SF2D_OK;
   }
-  using TileFn = void (*)(sf2d::Params, int, int, int);
+  using TileFn = void (*)(sf2d::Params, int, int, int, int);
   TileFn tile_fn = nullptr;
   TileFn pml_fn = nullptr;   // tiles [pml_tile0, ntiles) hold the CPML layer's elements
   int pml_tile0 = 0;
@@ -213,58 +219,53 @@ struct sf2d_solver {
     if (e != cudaSuccess && launch_error == cudaSuccess) launch_error = e;
   }
   cudaError_t launch_error = cudaSuccess;
-  void launch_tile(bool record_prev, int stage, int first = 0) {
+  // kstep: steps since the counter on the device was last advanced
+  void launch_tile(bool record_prev, int stage, int first, int kstep) {
     const int rp = record_prev ? 1 : 0;
     const int nplain = pml_tile0 - first;
     if (side) {
       cudaEventRecord(ev_fork, stream);
       cudaStreamWaitEvent(side, ev_fork, 0);
-      pml_fn<<<T.ntiles - pml_tile0, pml_nt, pml_smem, side>>>(pml_params(), rp, stage, pml_tile0);
+      pml_fn<<<T.ntiles - pml_tile0, pml_nt, pml_smem, side>>>(pml_params(), rp, stage, pml_tile0, kstep);
       cudaEventRecord(ev_join, side);
-      if (nplain > 0) tile_fn<<<nplain, nt, smem, stream>>>(P, rp, stage, first);
+      if (nplain > 0) tile_fn<<<nplain, lane_nt, smem, stream>>>(P, rp, stage, first, kstep);
       cudaStreamWaitEvent(stream, ev_join, 0);
       return;
     }
-    if (nplain > 0) launch_pdl(tile_fn, nplain, nt, smem, P, rp, stage, first);
-    if (pml_tile0 < T.ntiles) {
-      if (pml_fn)
-        pml_fn<<<T.ntiles - pml_tile0, pml_nt, pml_smem, stream>>>(pml_params(), rp, stage, pml_tile0);
-      else
-        tile_fn<<<T.ntiles - pml_tile0, nt, smem, stream>>>(P, rp, stage, pml_tile0);
-    }
+    if (nplain > 0) launch_pdl(tile_fn, nplain, lane_nt, smem, P, rp, stage, first, kstep);
+    if (pml_tile0 < T.ntiles)
+      pml_fn<<<T.ntiles - pml_tile0, pml_nt, pml_smem, stream>>>(pml_params(), rp, stage, pml_tile0, kstep);
   }
   // the early tiles [0, late_tile0) on stream s
-  void launch_early(cudaStream_t s, bool record_prev, int stage) {
-    if (late_tile0 > 0) tile_fn<<<late_tile0, nt, smem, s>>>(P, record_prev ? 1 : 0, stage, 0);
+  void launch_early(cudaStream_t s, bool record_prev, int stage, int kstep) {
+    if (late_tile0 > 0) tile_fn<<<late_tile0, lane_nt, smem, s>>>(P, record_prev ? 1 : 0, stage, 0, kstep);
   }
   // tile-kernel launches of one stage of launch_tile(first)
   int tile_launches(int first) const {
     return (pml_tile0 - first > 0) + (pml_tile0 < T.ntiles);
   }
-  void launch_shared(int stage) {
-    const int nb = std::max(1, (P.nshared + sf2d::SHARED_NT - 1) / sf2d::SHARED_NT);
-    const int last = stage == nstage - 1 ? 1 : 0;
+  void launch_shared(int stage, int kstep) {
+    if (P.nshared == 0) return;
+    const int nb = (P.nshared + sf2d::SHARED_NT - 1) / sf2d::SHARED_NT;
     if (lddrk)
-      launch_pdl(sf2d::k_elastic_shared<true, false>, nb, sf2d::SHARED_NT, 0, P, stage, last);
+      launch_pdl(sf2d::k_elastic_shared<true, false>, nb, sf2d::SHARED_NT, 0, P, stage, kstep);
     else if (kern)
-      launch_pdl(sf2d::k_elastic_shared<false, true>, nb, sf2d::SHARED_NT, 0, P, stage, last);
+      launch_pdl(sf2d::k_elastic_shared<false, true>, nb, sf2d::SHARED_NT, 0, P, stage, kstep);
     else
-      launch_pdl(sf2d::k_elastic_shared<false, false>, nb, sf2d::SHARED_NT, 0, P, stage, last);
+      launch_pdl(sf2d::k_elastic_shared<false, false>, nb, sf2d::SHARED_NT, 0, P, stage, kstep);
   }
-  int launch_step(bool record_prev) {
+  // the k-th step of a chunk
+  void launch_step(int k) {
     for (int st = 0; st < nstage; ++st) {
-      launch_tile(record_prev && st == 0, st);
-      launch_shared(st);
+      launch_tile(k > 0 && st == 0, st, 0, k);
+      launch_shared(st, k);
     }
-    return SF2D_OK;
   }
-  int launch_receivers() {
-    if (nrec > 0) launch_pdl(sf2d::k_receivers, (nrec + 127) / 128, 128, 0, P);
-    return SF2D_OK;
-  }
+  // after n steps: their last receiver samples, the step counter
+  void launch_advance(int n) { launch_pdl(sf2d::k_advance, 1, 256, 0, P, n); }
   int launch_chunk(int n) {
-    for (int k = 0; k < n; ++k) launch_step(k > 0);
-    launch_receivers();
+    for (int k = 0; k < n; ++k) launch_step(k);
+    launch_advance(n);
     if (launch_error != cudaSuccess) {
       const cudaError_t e = launch_error;
       launch_error = cudaSuccess;
@@ -283,6 +284,69 @@ struct sf2d_solver {
   }
 };
 
+
+namespace sf2d {
+// Kernel sums of an adjoint solver to the reference's element layout on the
+// device, with save_kernels_elastic's scaling (save_adjoint_kernels.f90:134-141):
+// one thread per element point, so that the host only receives the arrays.
+// (Gathering and scaling them on the host took as long as 100 steps of a
+// 64,000-element mesh.)
+struct KernelScale {
+  int nspec = 0;
+  float *mod = nullptr;   // [3][point]: rho, kappa, mu
+  float *out = nullptr;   // [3][point]: the scaled kernels
+  int *lane = nullptr;    // first row of each element
+  int *point = nullptr;   // device point of each element point
+  // Allocates through `alloc(void **, bytes)` and uploads; point arrays in
+  // reference layout.
+  template <typename Alloc>
+  int prepare(const sf2d_solver *A, int nspec_, const int *ibool, const float *rho, const float *kappa,
+              const float *mu, Alloc alloc);
+  // Kernels to host arrays, after the work queued on A's stream.
+  int fetch(const sf2d_solver *A, float dt, float *rho_kl, float *kappa_kl, float *mu_kl) const;
+};
+static __global__ void k_scale_kernels(KernelScale K, const float2 *kmu, const float *rho_glob, float dt) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, n = 25 * K.nspec;
+  if (p >= n) return;
+  const int q = p % 25, r = K.lane[p / 25] + q / 5;
+  const float2 km = kmu[(static_cast<size_t>(r >> 5) * 5 + q % 5) * 32 + (r & 31)];
+  const size_t sn = static_cast<size_t>(n);
+  K.out[p] = -K.mod[p] * dt * rho_glob[K.point[p]];
+  K.out[sn + p] = -K.mod[sn + p] * dt * km.x;
+  K.out[2 * sn + p] = -2.f * K.mod[2 * sn + p] * dt * km.y;
+}
+template <typename Alloc>
+int KernelScale::prepare(const sf2d_solver *A, int nspec_, const int *ibool, const float *rho, const float *kappa,
+                         const float *mu, Alloc alloc) {
+  nspec = nspec_;
+  const size_t n = static_cast<size_t>(nspec) * NGLL2;
+  std::vector<int> r(nspec), pt(n);
+  for (int s = 0; s < nspec; ++s) r[A->T.elem_order[s]] = A->slot_lane[s];
+  for (size_t p = 0; p < n; ++p) pt[p] = A->T.glob2dev[ibool[p]];
+  int rc;
+  if ((rc = alloc(reinterpret_cast<void **>(&mod), 3 * n * sizeof(float))) ||
+      (rc = alloc(reinterpret_cast<void **>(&out), 3 * n * sizeof(float))) ||
+      (rc = alloc(reinterpret_cast<void **>(&lane), r.size() * sizeof(int))) ||
+      (rc = alloc(reinterpret_cast<void **>(&point), n * sizeof(int))))
+    return rc;
+  SF2D_CUDA(cudaMemcpy(mod, rho, n * sizeof(float), cudaMemcpyHostToDevice));
+  SF2D_CUDA(cudaMemcpy(mod + n, kappa, n * sizeof(float), cudaMemcpyHostToDevice));
+  SF2D_CUDA(cudaMemcpy(mod + 2 * n, mu, n * sizeof(float), cudaMemcpyHostToDevice));
+  SF2D_CUDA(cudaMemcpy(lane, r.data(), r.size() * sizeof(int), cudaMemcpyHostToDevice));
+  SF2D_CUDA(cudaMemcpy(point, pt.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+  return SF2D_OK;
+}
+inline int KernelScale::fetch(const sf2d_solver *A, float dt, float *rho_kl, float *kappa_kl, float *mu_kl) const {
+  const size_t n = static_cast<size_t>(nspec) * NGLL2;
+  k_scale_kernels<<<static_cast<unsigned>((n + 255) / 256), 256, 0, A->stream>>>(*this, A->P.kmu_kl, A->P.rho_kl_glob, dt);
+  SF2D_CUDA(cudaGetLastError());
+  SF2D_CUDA(cudaMemcpyAsync(rho_kl, out, n * sizeof(float), cudaMemcpyDeviceToHost, A->stream));
+  SF2D_CUDA(cudaMemcpyAsync(kappa_kl, out + n, n * sizeof(float), cudaMemcpyDeviceToHost, A->stream));
+  SF2D_CUDA(cudaMemcpyAsync(mu_kl, out + 2 * n, n * sizeof(float), cudaMemcpyDeviceToHost, A->stream));
+  SF2D_CUDA(cudaStreamSynchronize(A->stream));
+  return SF2D_OK;
+}
+}  // namespace sf2d
 
 // Builds a solver; `kern` selects the adjoint variant that accumulates
 // sensitivity kernels against forward displacement frames.

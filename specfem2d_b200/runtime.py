@@ -182,7 +182,7 @@ def tiling_stats(db, tile_elems: int = 64):
                                tile_elems, out)
     if rc != 0:
         raise SF2DError(rc, "tiling invariant violated")
-    keys = ["ntiles", "nshared", "max_local", "max_elems", "max_colours", "n_interior", "n_slots", "reserved"]
+    keys = ["ntiles", "nshared", "max_local", "max_elems", "max_colours", "n_interior", "n_slots", "max_phases"]
     return dict(zip(keys, [int(x) for x in out]))
 
 

@@ -1,0 +1,110 @@
+"""Tiles by rows: local numbering, assembly phases and kernels on meshes whose
+elements do not share one orientation, and at tile sizes around one warp's
+elements.
+
+Half of the elements are turned by 180 degrees (their GLL arrays reversed, the
+mapping derivatives negated): the same mesh and medium, but neighbours hold
+common points at positions of one class, so that a tile needs more than the
+four assembly phases of a structured mesh.  The reference is the oracle on the
+mesh as it was; tolerance 1e-5 relative L2, the repository's bound for
+seismograms and displacement, and for kernels the FP32 oracle's own distance
+from FP64 (at least 1e-5)."""
+import copy
+
+import numpy as np
+import pytest
+
+from fwi_case import Case
+from helpers import rel_l2
+
+
+def turned(db, seed=0):
+    out = copy.copy(db)
+    t = np.random.default_rng(seed).random(db.nspec) < 0.5
+
+    def rev(a, sign=1.0):
+        a = np.array(a)
+        a[t] = sign * a[t][:, ::-1, ::-1]
+        return a
+
+    out.ibool = rev(db.ibool).astype(np.int32)
+    for k in ("xix", "xiz", "gammax", "gammaz"):
+        setattr(out, k, rev(getattr(db, k), -1.0))
+    for k in ("jacobian", "rhostore", "kappastore", "mustore", "rho_vpstore", "rho_vsstore"):
+        setattr(out, k, rev(getattr(db, k)))
+    if db.atten is not None:
+        out.atten = {k: rev(v) for k, v in db.atten.items()}
+    if db.aniso is not None:
+        out.aniso = {k: (v if k == "ispec" else rev(v)) for k, v in db.aniso.items()}
+    ts, tr = t[db.source_ispec], t[db.rec_ispec]
+    out.sourcearrays = np.array(db.sourcearrays)
+    out.sourcearrays[ts] = db.sourcearrays[ts][:, ::-1, ::-1]
+    out.hxir, out.hgammar = np.array(db.hxir), np.array(db.hgammar)
+    out.hxir[tr], out.hgammar[tr] = db.hxir[tr][:, ::-1], db.hgammar[tr][:, ::-1]
+    return out
+
+
+def _db(physics, nstep):
+    c = Case(nstep=nstep, qmu=40.0 if physics.startswith("visco") else None)
+    db = c.start_db()
+    if physics == "aniso":
+        f32 = np.float32
+        k, m = db.kappastore, db.mustore
+        db.aniso = {"ispec": np.arange(db.nspec) % 3 == 0, "c11": (1.1 * (k + m)).astype(f32),
+                    "c13": (0.9 * (k - m)).astype(f32), "c15": (0.02 * k).astype(f32), "c33": (k + m).astype(f32),
+                    "c35": (-0.01 * k).astype(f32), "c55": (1.05 * m).astype(f32)}
+    return db
+
+
+@pytest.mark.parametrize("tile_elems", [1, 5, 16, 33, 64, 256])
+def test_row_tiles_of_a_mesh_without_orientation(tile_elems):
+    from specfem2d_b200 import runtime
+
+    db = _db("iso", 10)
+    assert runtime.tiling_stats(db, tile_elems)["max_phases"] <= 4
+    st = runtime.tiling_stats(turned(db), tile_elems)
+    assert st["max_phases"] <= 16 and (tile_elems == 1 or st["max_phases"] >= 4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("physics,tile_elems", [("iso", 1), ("iso", 17), ("iso", 32), ("iso", 256), ("aniso", 31),
+                                                ("visco", 16), ("visco", 48), ("visco mixed", 32)])
+def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
+    import oracle
+    from specfem2d_b200.runtime import ElasticSolver
+
+    n = 400
+    db = _db(physics, n)
+    if physics == "visco mixed":
+        # coefficients that differ inside the elements: one set per point
+        for k in ("a1", "b1", "a2", "b2"):
+            db.atten[k] = (db.atten[k] * (1.0 + 1e-3 * (np.arange(25).reshape(5, 5) % 2))[None, :, :, None]).astype(np.float32)
+    s = ElasticSolver(turned(db), tile_elems=tile_elems)
+    seis = s.run(n)
+    o = oracle.Oracle(db, 4)
+    ref = o.run(n)
+    assert rel_l2(seis, ref) < 1e-5
+    assert rel_l2(s.get_fields()[0], o.displ) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("physics", ["iso", "visco"])
+def test_lane_gradient_on_a_mesh_without_orientation(physics):
+    import oracle
+    from specfem2d_b200.fwi import FWIGradient
+
+    n = 300
+    db = _db(physics, n)
+    t = np.arange(n)[None, :, None] / n
+    rng = np.random.default_rng(5)
+    adj = np.sin(2 * np.pi * rng.uniform(2, 6, (len(db.rec_ispec), 1, 2)) * t) * np.sin(np.pi * t) ** 2
+    tdb = turned(db)
+    g = FWIGradient(tdb, 70)
+    g.forward()
+    k = g.backward(adj)
+    flip = (tdb.ibool != db.ibool).any(axis=(1, 2))
+    o32, o64 = (oracle.adjoint_kernels(db, adj, checkpoint_every=70, precision=p)[2:] for p in (4, 8))
+    for got, r32, r64 in zip(k, o32, o64):
+        got = np.array(got)
+        got[flip] = got[flip][:, ::-1, ::-1]
+        assert rel_l2(got, r64) < max(1e-5, 1.5 * rel_l2(r32, r64))
