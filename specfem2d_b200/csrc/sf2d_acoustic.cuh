@@ -287,6 +287,7 @@ template <int NT, bool LDDRK>
 __global__ void __launch_bounds__(NT, 768 / NT)
     k_acoustic_pml_tile(const AcParams A, int stage, int tile0, int kstep) {
   extern __shared__ __align__(16) unsigned char smem[];
+  wait_previous_kernel();
   const TileInfo &ti = A.tiles[tile0 + blockIdx.x];
   const int tid = threadIdx.x;
   const int n_int = ti.n_int;
@@ -532,11 +533,21 @@ __global__ void __launch_bounds__(NT, 768 / NT)
 template <bool LDDRK>
 __global__ void __launch_bounds__(SHARED_NT) k_acoustic_shared(const AcParams A, int stage, int kstep) {
   const int s = blockIdx.x * SHARED_NT + threadIdx.x;
+  int k0 = 0, k1 = 0;
+  float rm = 0.f;
+  uint8_t m = 0;
+  if (s < A.nshared) {
+    k0 = __ldg(A.shp_off + s);
+    k1 = __ldg(A.shp_off + s + 1);
+    rm = __ldg(A.rmass + A.shared_begin + s);
+    m = __ldg(A.free_mask + A.shared_begin + s);
+  }
+  wait_previous_kernel();
+  allow_next_kernel();
   const int step = *A.d_step + kstep;
   if (s < A.nshared) {
     const int g = A.shared_begin + s;
     float p = A.p[g], pd = A.pd[g];
-    const uint8_t m = A.free_mask[g];
     if (!LDDRK) {
       const float pdd0 = A.pdd[g];
       if (A.pold)
@@ -551,8 +562,8 @@ __global__ void __launch_bounds__(SHARED_NT) k_acoustic_shared(const AcParams A,
       pd = 0.f;
     }
     float acc = 0.f;
-    for (int k = A.shp_off[s]; k < A.shp_off[s + 1]; ++k) acc += A.partial[k];
-    float pdd = acc * A.rmass[g];
+    for (int k = k0; k < k1; ++k) acc += A.partial[k];
+    float pdd = acc * rm;
     if (!LDDRK) {
       pd = newmark_veloc(pd, pdd, A.dto2);
     } else {
@@ -656,11 +667,16 @@ __global__ void k_cpl_pml_solid(const CplPml C, const float *p, const float *pd,
 // records step *d_step + kstep for every fluid receiver (launched after the last
 // stage of every step)
 static __global__ void k_acoustic_receivers(const AcParams A, int kstep) {
+  wait_previous_kernel();
+  allow_next_kernel();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < A.nrec) record_receiver_ac(A, r, *A.d_step + kstep);
 }
 
 // after n steps: the step counter
-static __global__ void k_acoustic_advance(const AcParams A, int n) { *A.d_step += n; }
+static __global__ void k_acoustic_advance(const AcParams A, int n) {
+  wait_previous_kernel();
+  *A.d_step += n;
+}
 
 }  // namespace sf2d

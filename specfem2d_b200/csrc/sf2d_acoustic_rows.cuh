@@ -97,6 +97,7 @@ __global__ void __maxnreg__(AC_ROW_REGS) k_acoustic_rows(const AcParams A, int s
   for (int l = tid; l < n_int; l += NT) cp_async4(s_rm + l, A.rmass + int_begin + l);
   cp_async_commit();
   for (int k = tid; k < 60; k += NT) s_h[k] = k < 55 ? A.hconst[k < 50 ? k : k + 5] : A.hsum[k - 55];
+  wait_previous_kernel();
   // fluid receivers are recorded by k_acoustic_receivers after each step: their
   // double-precision gradient would hold registers through the whole tile
   const int step = *A.d_step + kstep;

@@ -147,6 +147,14 @@ struct sf2d_coupled {
   // the fluid's CPML tiles beside the others, as the solid's (sf2d_solver::launch_tile)
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // on the run's stream, as the solid's step kernels: a step of a small ocean is
+  // a chain of six short kernels (121 x 67 elements: 25.0 -> 20.8 us a step,
+  // smaller tiles included)
+  cudaError_t launch_error = cudaSuccess;
+  template <typename F, typename... A_>
+  void launch_pdl(F fn, int grid, int block, size_t smem_bytes, A_... args) {
+    sf2d::launch_pdl(stream(), launch_error, fn, grid, block, smem_bytes, args...);
+  }
   void launch_ac_tile(int stage, int kstep) {
     cudaStream_t s = stream();
     if (side) {
@@ -158,16 +166,16 @@ struct sf2d_coupled {
       cudaStreamWaitEvent(s, ev_join, 0);
       return;
     }
-    if (pml_tile0 > 0) tile_fn<<<pml_tile0, lane_nt, smem, s>>>(A, stage, 0, kstep);
+    if (pml_tile0 > 0) launch_pdl(tile_fn, pml_tile0, lane_nt, smem, A, stage, 0, kstep);
     if (pml_tile0 < T.ntiles) pml_fn<<<T.ntiles - pml_tile0, nt, pml_smem, s>>>(A, stage, pml_tile0, kstep);
   }
   void launch_ac_shared(int stage, int kstep) {
     if (A.nshared == 0) return;
     const int nb = (A.nshared + sf2d::SHARED_NT - 1) / sf2d::SHARED_NT;
     if (lddrk)
-      sf2d::k_acoustic_shared<true><<<nb, sf2d::SHARED_NT, 0, stream()>>>(A, stage, kstep);
+      launch_pdl(sf2d::k_acoustic_shared<true>, nb, sf2d::SHARED_NT, 0, A, stage, kstep);
     else
-      sf2d::k_acoustic_shared<false><<<nb, sf2d::SHARED_NT, 0, stream()>>>(A, stage, kstep);
+      launch_pdl(sf2d::k_acoustic_shared<false>, nb, sf2d::SHARED_NT, 0, A, stage, kstep);
   }
   void launch_cpl_fluid(int stage) {
     if (cpl_fluid.n == 0) return;
@@ -207,7 +215,7 @@ struct sf2d_coupled {
       cudaEventRecord(ev_rec_done, side);
       rec_pending = true;
     } else {
-      sf2d::k_acoustic_receivers<<<nb, 128, 0, stream()>>>(A, kstep);
+      launch_pdl(sf2d::k_acoustic_receivers, nb, 128, 0, A, kstep);
     }
   }
   void join_ac_receivers() {
@@ -252,8 +260,15 @@ struct sf2d_coupled {
   int launch_chunk(int n) {
     for (int k = 0; k < n; ++k) launch_step(k);
     join_ac_receivers();
-    sf2d::k_acoustic_advance<<<1, 1, 0, stream()>>>(A, n);
+    launch_pdl(sf2d::k_acoustic_advance, 1, 1, 0, A, n);
     if (el) el->launch_advance(n);
+    cudaError_t e = launch_error;
+    launch_error = cudaSuccess;
+    if (el && el->launch_error != cudaSuccess) {
+      if (e == cudaSuccess) e = el->launch_error;
+      el->launch_error = cudaSuccess;
+    }
+    if (e != cudaSuccess) return sf2d::fail(SF2D_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     SF2D_CUDA(cudaGetLastError());
     return SF2D_OK;
   }
@@ -412,7 +427,7 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   // ---- fluid tiling and per-slot data
   if (ad->tile_elems > 256) return fail(SF2D_ERR_INVALID, "fluid tiling: tile_elems must be in [1, 256]");
   // five threads an element: 128 elements fit a block and its registers
-  const int te = std::min(ad->tile_elems > 0 ? ad->tile_elems : 32, 128);
+  const int te = tiles_for(std::min(ad->tile_elems > 0 ? ad->tile_elems : 32, 128), ad->nspec);
   // the fluid layer's tiles are a quarter of the size: there are few of them
   // (one wave), so the shorter per-tile latency sets the layer kernel's time
   const int group_te[2] = {te, std::max(4, (ad->tile_elems > 0 ? ad->tile_elems : 32) / 4)};

@@ -202,9 +202,11 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // before it in the stream still runs; griddepcontrol.wait then blocks until
 // that kernel has completed and its writes are visible, so every read of the
 // previous kernel's results comes after it.  launch_dependents lets the next
-// kernel be scheduled once all of this kernel's CTAs have started (the short
+// kernel be scheduled once all of this kernel's CTAs have started: the short
 // shared-point and receiver kernels call it, so the next step's tiles start as
-// they drain).  Both are no-ops for a kernel launched without the attribute.
+// they drain.  (A tile kernel that calls it costs 4 to 10 % per step from 80 x 60
+// to 1000 x 400 elements: the waiting CTAs sit beside the tiles.)
+// Both are no-ops for a kernel launched without the attribute.
 __device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
@@ -696,9 +698,16 @@ __global__ void __launch_bounds__(NT, 768 / NT)
 
 template <bool LDDRK, bool KERN>
 __global__ void __launch_bounds__(SHARED_NT) k_elastic_shared(const Params P, int stage, int kstep) {
+  const int s = blockIdx.x * SHARED_NT + threadIdx.x;
+  int k0 = 0, k1 = 0;
+  float2 rm = make_float2(0.f, 0.f);
+  if (s < P.nshared) {
+    k0 = __ldg(P.shp_off + s);
+    k1 = __ldg(P.shp_off + s + 1);
+    rm = __ldg(P.rmass + P.shared_begin + s);
+  }
   wait_previous_kernel();
   allow_next_kernel();
-  const int s = blockIdx.x * SHARED_NT + threadIdx.x;
   const int step = *P.d_step + kstep;
   if (s < P.nshared && !(P.shared_member && P.member_status[P.shared_member[s]])) {
     const int g = P.shared_begin + s;
@@ -715,12 +724,11 @@ __global__ void __launch_bounds__(SHARED_NT) k_elastic_shared(const Params P, in
       v = make_float2(0.f, 0.f);
     }
     float2 acc = make_float2(0.f, 0.f);
-    for (int k = P.shp_off[s]; k < P.shp_off[s + 1]; ++k) {
+    for (int k = k0; k < k1; ++k) {
       const float2 p = P.partial[k];
       acc.x += p.x;
       acc.y += p.y;
     }
-    const float2 rm = P.rmass[g];
     const float2 a = make_float2(acc.x * rm.x, acc.y * rm.y);
     if (!LDDRK) {
       v.x = v.x + P.dto2 * a.x;
