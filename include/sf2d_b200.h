@@ -87,9 +87,11 @@ typedef struct {
   /* time stepping */
   int nstep;                                 /* length of stf and of the seismogram buffer */
   float deltat, deltatover2, deltatsquareover2;
-  int tile_elems;                            /* elements per tile, 0 = default (64) */
-  int threads_per_block;                     /* 128, 250, 256 or 512; 0 = default (256); 250 keeps
-                                                each thread on one GLL position of every element */
+  int tile_elems;                            /* elements per tile (1 to 256; 128 at most and fewer on small
+                                                meshes are used outside CPML layers), 0 = default (64) */
+  int threads_per_block;                     /* of the CPML tiles' kernel: 128, 250, 256 or 512; 0 = default
+                                                (256); 250 keeps each thread on one GLL position of every
+                                                element.  Other tiles take five threads per element. */
   /* time scheme: 1 (or 0) Newmark, 2 LDDRK with 6 stages (update_displacement_LDDRK.F90);
    * stf holds nstage values per step: stf[isrc][it][stage] */
   int time_scheme;
@@ -325,7 +327,7 @@ int sf2d_smooth(int nspec, const float *x, const float *z, const float *jacobian
  * its invariants (one device id per point, local ibool consistent with
  * ibool, colours conflict-free, shared-point slots complete and in tile
  * order).  out8 = [ntiles, nshared, max local points, max elements per tile,
- * max colours, interior points, partial-sum slots, 0].  Returns 0 when every
+ * max colours, interior points, partial-sum slots, max assembly phases by rows].  Returns 0 when every
  * invariant holds, a negative code naming the first that fails otherwise.
  * No reference counterpart (the reference assembles with atomics). */
 int sf2d_tiling_stats(int nspec, int nglob, const int *ibool, const double *centroid_xz, int tile_elems,

@@ -4,7 +4,7 @@ A batch is packed into one disconnected mesh: member m's elements, global
 points, absorbing points, sources and receivers are appended with offsets
 (its element ids shifted by the elements before it, its global ids by the
 points before it), and its coordinates are shifted far apart along x so the
-Morton-ordered tiles of the tiler never mix members.  The tile-staged kernels
+tiler, which cuts connected parts one by one, never mixes members in a tile.  The tile-staged kernels
 need no change: every tile belongs to one member, shared points stay inside a
 member, and the per-step launch count is that of a single run.  This is the
 GPU counterpart of the reference's NUMBER_OF_SIMULTANEOUS_RUNS

@@ -132,7 +132,7 @@ std::vector<T> transpose(const U *a, int n1, int n2) {
   return out;
 }
 
-// Element centres for the tiler's Morton order.  The reference hands the GPU
+// Element centres for the tiler's bisection.  The reference hands the GPU
 // no coordinates, so they are rebuilt from the mapping derivatives: x_xi =
 // gammaz J, z_xi = -gammax J, x_gamma = -xiz J, z_gamma = xix J with J =
 // 1/(xix gammaz - xiz gammax), integrated along GLL lines through the
