@@ -341,16 +341,31 @@ std::string build_tiling(int nspec, int nglob, const int *ibool, const double *c
           ti.ncol = std::max(ti.ncol, p + 1);
         }
     } else {
-      used.assign(nl, 0u);
-      cls.assign(ne, 0);
-      for (int k = 0; k < ne; ++k) {
-        uint32_t m = 0;
-        for (int q = 0; q < NGLL2; ++q) m |= used[lid[static_cast<size_t>(k) * NGLL2 + q]];
-        int c = 0;
-        while (c < MAX_COLOURS && (m >> c) & 1u) ++c;
-        if (c == MAX_COLOURS) return "element colouring needs more than 8 colours in a tile";
-        cls[k] = c;
-        for (int q = 0; q < NGLL2; ++q) used[lid[static_cast<size_t>(k) * NGLL2 + q]] |= 1u << c;
+      auto colour = [&](const std::vector<int> &seq) {
+        used.assign(nl, 0u);
+        cls.assign(ne, 0);
+        for (int k : seq) {
+          uint32_t m = 0;
+          for (int q = 0; q < NGLL2; ++q) m |= used[lid[static_cast<size_t>(k) * NGLL2 + q]];
+          int c = 0;
+          while (c < MAX_COLOURS && (m >> c) & 1u) ++c;
+          if (c == MAX_COLOURS) return false;
+          cls[k] = c;
+          for (int q = 0; q < NGLL2; ++q) used[lid[static_cast<size_t>(k) * NGLL2 + q]] |= 1u << c;
+        }
+        return true;
+      };
+      if (!colour(idx)) {
+        // elements numbered at random can use up the colours; along the tile's
+        // rows a structured mesh takes four or five whatever its numbering
+        if (centroid_xz)
+          std::sort(idx.begin(), idx.end(), [&](int a, int c) {
+            const size_t p = 2 * static_cast<size_t>(order[b + a]), r = 2 * static_cast<size_t>(order[b + c]);
+            if (key[p + 1] != key[r + 1]) return key[p + 1] < key[r + 1];
+            return key[p] != key[r] ? key[p] < key[r] : a < c;
+          });
+        if (!centroid_xz || !colour(idx)) return "element colouring needs more than 8 colours in a tile";
+        std::iota(idx.begin(), idx.end(), 0);
       }
       std::stable_sort(idx.begin(), idx.end(), [&](int a, int c) { return cls[a] < cls[c]; });
     }

@@ -2,6 +2,7 @@
 function include/sf2d_b200.h declares, and its tiler keeps its invariants."""
 import os
 import re
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
@@ -38,6 +39,27 @@ def test_tiling_invariants(tile_elems):
     assert st["ntiles"] == -(-db.nspec // tile_elems)
     assert st["n_interior"] + st["nshared"] == db.nglob
     assert st["max_colours"] <= 8
+
+
+@pytest.mark.parametrize("nx,nz,tile_elems,seed", [(16, 16, 256, 3908), (16, 16, 256, 6278), (16, 16, 64, 0),
+                                                   (40, 30, 32, 1)])
+def test_tiling_of_elements_numbered_at_random(nx, nz, tile_elems, seed):
+    """Which tiles a mesh is cut into must not decide whether it is accepted:
+    first-fit colouring in the elements' numbering needs a ninth colour for the
+    first two numberings."""
+    ib = np.zeros((nz, nx, 5, 5), dtype=np.int32)
+    for j in range(5):
+        for i in range(5):
+            ib[:, :, j, i] = (4 * np.arange(nz) + j)[:, None] * (4 * nx + 1) + 4 * np.arange(nx) + i
+    perm = np.random.default_rng(seed).permutation(nx * nz)
+    ib = ib.reshape(-1, 5, 5)[perm]
+    nglob = (4 * nx + 1) * (4 * nz + 1)
+    pts = np.arange(nglob)
+    coord = np.stack([pts % (4 * nx + 1), pts // (4 * nx + 1)], 1) / 4.0
+    db = SimpleNamespace(nspec=nx * nz, nglob=nglob, ibool=ib, coord=coord)
+    st = runtime.tiling_stats(db, tile_elems)
+    assert st["max_colours"] <= 8 and st["max_phases"] <= 4
+    assert st["n_interior"] + st["nshared"] == nglob
 
 
 def test_coupled_split_keeps_every_interface_point():
