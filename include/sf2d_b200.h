@@ -87,8 +87,8 @@ typedef struct {
   /* time stepping */
   int nstep;                                 /* length of stf and of the seismogram buffer */
   float deltat, deltatover2, deltatsquareover2;
-  int tile_elems;                            /* elements per tile (1 to 256; 128 at most and fewer on small
-                                                meshes are used outside CPML layers), 0 = default (64) */
+  int tile_elems;                            /* elements per tile (1 to 256; 128 at most outside CPML layers);
+                                                -n: up to n, fewer on small meshes; 0: as -64 */
   int threads_per_block;                     /* of the CPML tiles' kernel: 128, 250, 256 or 512; 0 = default
                                                 (256); 250 keeps each thread on one GLL position of every
                                                 element.  Other tiles take five threads per element. */

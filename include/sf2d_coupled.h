@@ -61,7 +61,7 @@ typedef struct {
   const int *rec_ispec;
   const double *hxir, *hgammar;              /* nrec*5 */
   const int *rec_global;                     /* index of each in the run's receiver list */
-  int tile_elems;                            /* 0 = 32 */
+  int tile_elems;                            /* as sf2d_elastic_desc's; 0: as -32 */
   /* CPML layer in the fluid (pml_region NULL = none), as in sf2d_elastic_desc;
    * edge points: pml_boundary_acoustic (pml_compute.f90:502-541) */
   const int *pml_region;

@@ -147,7 +147,7 @@ class NativeBatch:
     makes them).  checkpoint_every > 0 makes a gradient batch whose kernels
     come back per model, summed over its shots."""
 
-    def __init__(self, models, shots=None, shot_models=None, checkpoint_every: int = 0, tile_elems: int = 32,
+    def __init__(self, models, shots=None, shot_models=None, checkpoint_every: int = 0, tile_elems: int = 0,
                  threads_per_block: int = 256):
         import ctypes
 

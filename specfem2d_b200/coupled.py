@@ -15,7 +15,7 @@ import ctypes
 
 import numpy as np
 
-from .runtime import _check, _d, _f, _i, _seis_buffer, build_desc, load_library, time_desc
+from .runtime import _check, _d, _f, _i, _seis_buffer, build_desc, load_library, tile_hint, time_desc
 
 _vp = ctypes.c_void_p
 
@@ -186,7 +186,7 @@ def split(db):
     return sub, fluid, cpl, dict(solid_points=gl, fluid_points=ga)
 
 
-def coupled_descs(db, tile_elems: int = 32, threads_per_block: int = 256, fluid_tile_elems: int = 0,
+def coupled_descs(db, tile_elems: int = 0, threads_per_block: int = 256, fluid_tile_elems: int = 0,
                   fluid_threads_per_block: int = 0, pml_tile_elems: int = 0, pml_threads_per_block: int = 0):
     """The C descriptions of a coupled Database: (solid desc, fluid desc,
     coupling desc, arrays to keep alive, solid sub-Database or None, fluid
@@ -228,7 +228,7 @@ def coupled_descs(db, tile_elems: int = 32, threads_per_block: int = 256, fluid_
     a.sourcearrays, a.stf = f(fl["sourcearrays"]), f(fl["stf"])
     a.nrec, a.rec_ispec = len(fl["rec_ispec"]), i(fl["rec_ispec"])
     a.hxir, a.hgammar, a.rec_global = dd(fl["hxir"]), dd(fl["hgammar"]), i(fl["rec_global"])
-    a.tile_elems = fluid_tile_elems or tile_elems
+    a.tile_elems = tile_hint(fluid_tile_elems or tile_elems)
     a.threads_per_block = fluid_threads_per_block
     fp = fl["pml"]
     if fp is not None:
@@ -257,7 +257,7 @@ def coupled_descs(db, tile_elems: int = 32, threads_per_block: int = 256, fluid_
 class CoupledSolver:
     """Device-resident coupled fluid-solid solver for one Database."""
 
-    def __init__(self, db, tile_elems: int = 32, threads_per_block: int = 256, fluid_tile_elems: int = 0,
+    def __init__(self, db, tile_elems: int = 0, threads_per_block: int = 256, fluid_tile_elems: int = 0,
                  fluid_threads_per_block: int = 0, pml_tile_elems: int = 0, pml_threads_per_block: int = 0):
         """Tile sizes and threads per CTA of the solid; the fluid's default to the same."""
         lib = _lib()
@@ -407,7 +407,7 @@ class CoupledKernels:
 
     Newmark, Stacey or free edges (no CPML)."""
 
-    def __init__(self, db, checkpoint_every: int = 200, tile_elems: int = 32, threads_per_block: int = 256):
+    def __init__(self, db, checkpoint_every: int = 200, tile_elems: int = 0, threads_per_block: int = 256):
         if int(db.time_scheme) != 1:
             raise ValueError("the kernel run is implemented for the Newmark scheme")
         if getattr(db, "pml", None) is not None:

@@ -426,11 +426,10 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
 
   // ---- fluid tiling and per-slot data
   if (ad->tile_elems > 256) return fail(SF2D_ERR_INVALID, "fluid tiling: tile_elems must be in [1, 256]");
-  // five threads an element: 128 elements fit a block and its registers
-  const int te = tiles_for(std::min(ad->tile_elems > 0 ? ad->tile_elems : 32, 128), ad->nspec);
+  const int te = row_tile_elems(ad->tile_elems, 32, ad->nspec);
   // the fluid layer's tiles are a quarter of the size: there are few of them
   // (one wave), so the shorter per-tile latency sets the layer kernel's time
-  const int group_te[2] = {te, std::max(4, (ad->tile_elems > 0 ? ad->tile_elems : 32) / 4)};
+  const int group_te[2] = {te, std::max(4, tile_hint(ad->tile_elems, 32) / 4)};
   std::string err = build_tiling(ad->nspec, ad->nglob, ad->ibool, ad->centroid_xz, te, C->T,
                                  pml_ac ? group.data() : nullptr, pml_ac ? 2 : 1, pml_ac ? group_te : nullptr, 1);
   if (!err.empty()) return fail(SF2D_ERR_INVALID, "fluid tiling: " + err);

@@ -109,9 +109,8 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   auto *S = new sf2d_solver();
   std::unique_ptr<sf2d_solver> guard(S);
   if (d->tile_elems > 256) return fail(SF2D_ERR_INVALID, "tiling: tile_elems must be in [1, 256]");
-  // five threads an element and at most 96 registers a thread: 128 elements fit the register file
-  const int te = tiles_for(std::min(d->tile_elems > 0 ? d->tile_elems : 64, 128), d->nspec);
-  const int group_te[3] = {te, te, d->pml_tile_elems > 0 ? d->pml_tile_elems : d->tile_elems > 0 ? d->tile_elems : 64};
+  const int te = row_tile_elems(d->tile_elems, 64, d->nspec);
+  const int group_te[3] = {te, te, d->pml_tile_elems > 0 ? d->pml_tile_elems : tile_hint(d->tile_elems, 64)};
   std::string err = build_tiling(d->nspec, d->nglob, d->ibool, d->centroid_xz, te, S->T,
                                  grouped ? group.data() : nullptr, grouped ? 3 : 1, grouped ? group_te : nullptr,
                                  grouped ? 2 : 1);

@@ -294,7 +294,7 @@ void build_solver(const char *routine, FortranMesh &m) {
   d.deltat = m.dt;
   d.deltatover2 = m.dtover2;
   d.deltatsquareover2 = m.dtsq2;
-  d.tile_elems = 32;
+  d.tile_elems = -32;
   d.threads_per_block = 256;
   d.time_scheme = 1;
   d.nstage = 1;
@@ -479,7 +479,7 @@ void build_coupled(const char *routine, FortranMesh &m) {
   d.deltat = m.dt;
   d.deltatover2 = m.dtover2;
   d.deltatsquareover2 = m.dtsq2;
-  d.tile_elems = 32;
+  d.tile_elems = -32;
   d.threads_per_block = 256;
   d.time_scheme = 1;
   d.nstage = 1;
@@ -646,7 +646,7 @@ void build_coupled(const char *routine, FortranMesh &m) {
   a.hxir = f_hxir.data();
   a.hgammar = f_hgammar.data();
   a.rec_global = f_rec_global.data();
-  a.tile_elems = 32;
+  a.tile_elems = -32;
   std::vector<int> f_pml_region, f_pml_edge;
   std::vector<double> f_pml[6];
   if (m.pml) {

@@ -52,12 +52,25 @@ void launch_pdl(cudaStream_t stream, cudaError_t &first_error, F fn, int grid, i
 
 using TileKernel = void (*)(Params, int, int, int, int);
 
-// Elements per tile of a mesh (or domain) of n elements where `te` are asked
-// for: halved (to 8 at least) while the tiles would not give every SM one and
-// every other SM a second.  A step of a small mesh takes as long as one tile
-// does: 80 x 60 elements take 9.9 us with 150 tiles of 32 and 8.8 us with 300 of
-// 16; 233 x 147 elements (1071 tiles of 32) 17.9 us, and 19.1 us in tiles of 16.
-inline int tiles_for(int te, int n) {
+// Five threads an element and at most 96 registers a thread: 128 elements fit
+// a CTA and the register file.
+constexpr int MAX_ROW_ELEMS = 128;
+
+// A description's tile_elems: > 0 as given; -n "up to n"; 0 up to `standard`.
+inline int tile_hint(int asked, int standard) {
+  if (asked < 0) return -std::max(asked, -256);
+  return asked > 0 ? asked : standard;
+}
+
+// Elements per tile by rows of a mesh (or domain) of n elements.  A size that
+// is asked for is used; "up to" is halved (to 8 at least) while the tiles would
+// not give every SM one and every other SM a second.  A step of a small mesh
+// takes as long as one tile does: 80 x 60 elements take 9.9 us with 150 tiles of
+// 32 and 8.8 us with 300 of 16; 233 x 147 elements (1071 tiles of 32) 17.9 us,
+// and 19.1 us in tiles of 16.
+inline int row_tile_elems(int asked, int standard, int n) {
+  int te = std::min(tile_hint(asked, standard), MAX_ROW_ELEMS);
+  if (asked > 0) return te;
   while (te >= 16 && 2 * static_cast<long long>((n + te - 1) / te) < 3 * 148) te /= 2;
   return te;
 }

@@ -24,7 +24,7 @@ from .runtime import _check, _d, _f, build_desc, load_library
 
 
 class FWIGradient:
-    def __init__(self, db, checkpoint_every: int = 200, tile_elems: int = 32, threads_per_block: int = 256,
+    def __init__(self, db, checkpoint_every: int = 200, tile_elems: int = 0, threads_per_block: int = 256,
                  hessian: bool = False):
         """`hessian` also accumulates the approximate Hessian (see hessian())."""
         if int(db.time_scheme) != 1:

@@ -219,7 +219,13 @@ def member_norms_noalloc(field_ptr: int, offsets, stream: int = 0) -> np.ndarray
     return out
 
 
-def build_desc(db, tile_elems: int = 32, seismotype: int = 1, threads_per_block: int = 256,
+def tile_hint(tile_elems: int) -> int:
+    """The descriptions' tile_elems: a size as given, 0 (the default): up to 32
+    elements, fewer on meshes whose tiles of 32 would not fill the GPU."""
+    return tile_elems or -32
+
+
+def build_desc(db, tile_elems: int = 0, seismotype: int = 1, threads_per_block: int = 256,
                pml_tile_elems: int = 0, pml_threads_per_block: int = 0):
     """sf2d_elastic_desc for a setup Database; returns (desc, arrays kept alive)."""
     keep = []
@@ -265,7 +271,7 @@ def build_desc(db, tile_elems: int = 32, seismotype: int = 1, threads_per_block:
     d.nstep = db.nstep
     d.deltat, d.deltatover2, d.deltatsquareover2 = (float(db.deltat), float(db.deltatover2),
                                                     float(db.deltatsquareover2))
-    d.tile_elems = tile_elems
+    d.tile_elems = tile_hint(tile_elems)
     d.threads_per_block = threads_per_block
     d.pml_tile_elems, d.pml_threads_per_block = pml_tile_elems, pml_threads_per_block
     from .setup.solver_setup import ALPHA_LDDRK, BETA_LDDRK
@@ -303,7 +309,7 @@ def build_desc(db, tile_elems: int = 32, seismotype: int = 1, threads_per_block:
     return d, keep
 
 
-def time_desc(db, tile_elems: int = 32, threads_per_block: int = 256):
+def time_desc(db, tile_elems: int = 0, threads_per_block: int = 256):
     """sf2d_elastic_desc with no element: the time stepping and GLL members of
     `db` only (the solid side of a fluid-only coupled run)."""
     keep = []
@@ -321,7 +327,7 @@ def time_desc(db, tile_elems: int = 32, threads_per_block: int = 256):
     d.nstep = db.nstep
     d.deltat, d.deltatover2, d.deltatsquareover2 = (float(db.deltat), float(db.deltatover2),
                                                     float(db.deltatsquareover2))
-    d.tile_elems, d.threads_per_block = tile_elems, threads_per_block
+    d.tile_elems, d.threads_per_block = tile_hint(tile_elems), threads_per_block
     d.time_scheme = int(db.time_scheme)
     d.nstage = int(db.stf.shape[2])
     d.alpha_lddrk, d.beta_lddrk = f(ALPHA_LDDRK), f(BETA_LDDRK)
@@ -332,7 +338,7 @@ def time_desc(db, tile_elems: int = 32, threads_per_block: int = 256):
 class ElasticSolver:
     """Device-resident elastic solver (Newmark or LDDRK) for one Database."""
 
-    def __init__(self, db, tile_elems: int = 32, seismotype: int = 1, threads_per_block: int = 256,
+    def __init__(self, db, tile_elems: int = 0, seismotype: int = 1, threads_per_block: int = 256,
                  pml_tile_elems: int = 0, pml_threads_per_block: int = 0):
         lib = load_library()
         d, keep = build_desc(db, tile_elems, seismotype, threads_per_block, pml_tile_elems, pml_threads_per_block)

@@ -77,6 +77,7 @@ def test_tile_size_invariance(tromp, oracle_1500, tile_elems, threads):
     db, _ = tromp
     ref, d_or, v_or, v64 = oracle_1500
     sol = ElasticSolver(db, tile_elems=tile_elems, threads_per_block=threads)
+    assert sol.layout_info()["max_elems"] == tile_elems
     s = sol.run(1500)
     assert rel_l2(s, ref) < TOL
     d, v, _ = sol.get_fields()
@@ -138,11 +139,26 @@ def test_solvers_with_different_tile_sizes_coexist(tromp):
     db, _ = tromp
     big = ElasticSolver(db, tile_elems=128)
     small = ElasticSolver(db, tile_elems=8)
+    assert big.layout_info()["max_elems"] == 128 and small.layout_info()["max_elems"] == 8
     a = big.run(64)
     b = small.run(64)
     assert rel_l2(a, b) < TOL
     big.close()
     small.close()
+
+
+def test_tile_size_is_the_callers_and_otherwise_fits_the_mesh(tromp):
+    """A size that is asked for is used (128 at most); the default is 32, halved
+    until the 2,560 elements' tiles would fill every other SM twice."""
+    from specfem2d_b200.runtime import ElasticSolver
+
+    db, _ = tromp
+    for asked, used in ((16, 16), (32, 32), (100, 100), (256, 128), (0, 8)):
+        s = ElasticSolver(db, tile_elems=asked)
+        info = s.layout_info()
+        assert info["max_elems"] == used and info["ntiles"] == -(-db.nspec // used)
+        s.close()
+    assert ElasticSolver(db).layout_info()["max_elems"] == 8
 
 
 def test_initialize_device_selects_rank_modulo_devices(tromp):

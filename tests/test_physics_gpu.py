@@ -21,6 +21,8 @@ def _compare(db, nstep, **solver_kw):
     o = oracle.Oracle(db, 4)
     ref = o.run(nstep)
     sol = ElasticSolver(db, **solver_kw)
+    if "tile_elems" in solver_kw:
+        assert sol.layout_info()["max_elems"] == solver_kw["tile_elems"]
     s = sol.run(nstep)
     d, _, _ = sol.get_fields()
     return s, ref, d, o.displ

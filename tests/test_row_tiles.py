@@ -68,7 +68,8 @@ def test_row_tiles_of_a_mesh_without_orientation(tile_elems):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("physics,tile_elems", [("iso", 1), ("iso", 17), ("iso", 32), ("iso", 256), ("aniso", 31),
-                                                ("visco", 16), ("visco", 48), ("visco mixed", 32)])
+                                                ("aniso", 128), ("visco", 16), ("visco", 48), ("visco", 128),
+                                                ("visco mixed", 32)])
 def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
     import oracle
     from specfem2d_b200.runtime import ElasticSolver
@@ -80,6 +81,7 @@ def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
         for k in ("a1", "b1", "a2", "b2"):
             db.atten[k] = (db.atten[k] * (1.0 + 1e-3 * (np.arange(25).reshape(5, 5) % 2))[None, :, :, None]).astype(np.float32)
     s = ElasticSolver(turned(db), tile_elems=tile_elems)
+    assert s.layout_info()["max_elems"] == min(tile_elems, 128)
     seis = s.run(n)
     o = oracle.Oracle(db, 4)
     ref = o.run(n)
@@ -88,8 +90,9 @@ def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("physics", ["iso", "visco"])
-def test_lane_gradient_on_a_mesh_without_orientation(physics):
+@pytest.mark.parametrize("physics,tile_elems", [("iso", 0), ("iso", 33), ("iso", 128), ("visco", 0), ("visco", 64),
+                                                ("visco", 128)])
+def test_lane_gradient_on_a_mesh_without_orientation(physics, tile_elems):
     import oracle
     from specfem2d_b200.fwi import FWIGradient
 
@@ -99,7 +102,7 @@ def test_lane_gradient_on_a_mesh_without_orientation(physics):
     rng = np.random.default_rng(5)
     adj = np.sin(2 * np.pi * rng.uniform(2, 6, (len(db.rec_ispec), 1, 2)) * t) * np.sin(np.pi * t) ** 2
     tdb = turned(db)
-    g = FWIGradient(tdb, 70)
+    g = FWIGradient(tdb, 70, tile_elems=tile_elems)
     g.forward()
     k = g.backward(adj)
     flip = (tdb.ibool != db.ibool).any(axis=(1, 2))
