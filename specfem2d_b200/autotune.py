@@ -1,11 +1,12 @@
 """Autotuner for the tile-staged kernels and for packed batches.
 
-* ``autotune_elastic``: elements per tile x threads per CTA of a solid mesh.
-  Each candidate builds its tiling, runs a few warm-up steps, then times
-  `steps` single launches with CUDA events (sf2d_time_kernels) and keeps the
-  configuration with the smallest time per step (element kernel plus
-  shared-point kernel).  Candidates whose shared memory does not fit are
-  skipped.
+* ``autotune_elastic``: elements per tile of a solid mesh, and threads per CTA
+  of its CPML tiles where it has any (the other tiles take five threads an
+  element).  Each candidate builds its tiling, runs a few warm-up steps, then
+  times `steps` single launches with CUDA events (sf2d_time_kernels) and keeps
+  the configuration with the smallest time per step (element kernel plus
+  shared-point kernel).  Candidates whose shared memory does not fit, and those
+  whose tiles have been timed already, are skipped.
 * ``autotune_coupled``: fluid tile size and the solid CPML tiles' size and
   threads of a coupled mesh.  The solid and fluid kernels overlap on two
   streams, so each candidate is timed on whole graph-queued steps.
@@ -22,7 +23,7 @@ import time
 
 import numpy as np
 
-DEFAULT_TILES = (32, 48, 64, 96, 128)
+DEFAULT_TILES = (0, 32, 48, 64, 96, 128)  # 0: by the mesh's size
 DEFAULT_THREADS = (128, 256, 512)
 
 
@@ -31,7 +32,10 @@ def autotune_elastic(db, tiles=DEFAULT_TILES, threads=DEFAULT_THREADS, steps: in
     """Returns (best (tile_elems, threads), list of result dicts)."""
     from .runtime import ElasticSolver, SF2DError
 
-    results = []
+    pml = getattr(db, "pml", None)
+    if pml is None or not (np.asarray(pml["region"]) > 0).any():
+        threads = threads[:1]
+    results, seen = [], set()
     for te in tiles:
         for nt in threads:
             try:
@@ -40,14 +44,20 @@ def autotune_elastic(db, tiles=DEFAULT_TILES, threads=DEFAULT_THREADS, steps: in
                 results.append({"tile_elems": te, "threads": nt, "error": str(e)})
                 continue
             try:
+                info = sol.layout_info()
+                layout = (nt,) + tuple(info[k] for k in ("ntiles", "nshared", "max_elems", "threads_per_block"))
+                if layout in seen:
+                    continue
+                seen.add(layout)
                 sol.enqueue(warmup)
                 sol.synchronize(120)
                 ms = sol.time_kernels(steps)
-                info = sol.layout_info()
             finally:
                 sol.close()
-            r = {"tile_elems": te, "threads": nt, "tile_ms": ms[0], "shared_ms": ms[1], "step_ms": ms[2],
-                 "ntiles": info["ntiles"], "nshared": info["nshared"], "smem_bytes": info["smem_bytes"]}
+            r = {"tile_elems": te, "threads": nt, "max_elems": info["max_elems"],
+                 "threads_per_cta": info["threads_per_block"], "tile_ms": ms[0], "shared_ms": ms[1],
+                 "step_ms": ms[2], "ntiles": info["ntiles"], "nshared": info["nshared"],
+                 "smem_bytes": info["smem_bytes"]}
             results.append(r)
             if verbose:
                 print(json.dumps(r), flush=True)
@@ -69,7 +79,7 @@ def _time_steps(sol, steps: int, warmup: int) -> float:
     return (time.perf_counter() - t0) * 1e3 / steps
 
 
-def autotune_coupled(db, tile_elems: int = 32, threads: int = 256, fluid_tiles=(32, 64),
+def autotune_coupled(db, tile_elems: int = 0, threads: int = 256, fluid_tiles=(32, 64),
                      pml=((16, 128), (32, 256)), steps: int = 64, warmup: int = 8, verbose: bool = False):
     """Returns (best (fluid_tile_elems, pml_tile_elems, pml_threads), results) for a coupled Database."""
     from .coupled import CoupledSolver
