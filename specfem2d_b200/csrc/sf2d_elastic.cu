@@ -8,11 +8,11 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "sf2d_b200.h"
@@ -180,42 +180,71 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
       mat.push_back(make_float2(d->lambdastore[p], d->mustore[p]));
     }
   // attenuation coefficients: sets of equal values, named per element or, when
-  // some element mixes them, per point
-  std::vector<float4> att_sets;
+  // some element mixes them, per point; every point's own where those are more
+  // than MAX_POINT_SETS (sf2d_rows.cuh has both sides' times)
+  std::vector<float4> att_sets, att_coef;
   std::vector<int> att_eset, att_pset;
   if (atten) {
+    const size_t MAX_POINT_SETS = lddrk ? 16384 : 1024;
     const float *k0 = lddrk ? d->att_itau1 : d->att_a1, *k1 = lddrk ? d->att_itau2 : d->att_a2;
     const float *k2 = lddrk ? d->att_phi1 : d->att_b1, *k3 = lddrk ? d->att_phi2 : d->att_b2;
-    std::map<std::array<uint32_t, 12>, int> seen;
-    std::vector<int> pset(nq, 0);
-    std::array<uint32_t, 12> key{}, prev{};
-    int id = -1;
+    auto first = [&](int s, int q) { return (static_cast<size_t>(T.elem_order[s]) * NGLL2 + q) * 3; };
+    auto coef = [&](size_t p, int l) { return make_float4(k0[p + l], k1[p + l], k2[p + l], k3[p + l]); };
+    auto same = [&](size_t p, size_t r) {
+      return !std::memcmp(k0 + p, k0 + r, 12) && !std::memcmp(k1 + p, k1 + r, 12) && !std::memcmp(k2 + p, k2 + r, 12) &&
+             !std::memcmp(k3 + p, k3 + r, 12);
+    };
     bool mixed = false;
-    for (int s = 0; s < pml_slot0; ++s)
-      for (int q = 0; q < NGLL2; ++q) {
-        const size_t p = (static_cast<size_t>(T.elem_order[s]) * NGLL2 + q) * 3;
+    for (int s = 0; s < pml_slot0 && !mixed; ++s)
+      for (int q = 1; q < NGLL2; ++q) mixed |= !same(first(s, 0), first(s, q));
+    // the set of the point whose coefficients start at p, made if there is none
+    // (past MAX_POINT_SETS of them without looking for one)
+    struct Hash {
+      size_t operator()(const std::array<uint32_t, 12> &a) const {
+        uint64_t h = 1469598103934665603ull;
+        for (uint32_t x : a) h = (h ^ x) * 1099511628211ull;
+        return static_cast<size_t>(h ^ (h >> 29));
+      }
+    };
+    std::unordered_map<std::array<uint32_t, 12>, int, Hash> seen;
+    int id = -1;
+    size_t prev = 0;
+    auto set_of = [&](size_t p) {
+      if (id >= 0 && same(prev, p)) return id;
+      prev = p;
+      id = static_cast<int>(att_sets.size() / 3);
+      if (seen.size() <= MAX_POINT_SETS) {
+        std::array<uint32_t, 12> key;
         std::memcpy(&key[0], k0 + p, 12);
         std::memcpy(&key[3], k1 + p, 12);
         std::memcpy(&key[6], k2 + p, 12);
         std::memcpy(&key[9], k3 + p, 12);
-        if (id < 0 || key != prev) {
-          const auto it = seen.emplace(key, static_cast<int>(seen.size()));
-          id = it.first->second;
-          if (it.second) {
-            for (int l = 0; l < 3; ++l) att_sets.push_back(make_float4(k0[p + l], k1[p + l], k2[p + l], k3[p + l]));
-          }
-          prev = key;
-        }
-        pset[S->lane_index(s, q)] = id;
-        if (q > 0 && pset[S->lane_index(s, 0)] != id) mixed = true;
+        const auto it = seen.emplace(key, id);
+        id = it.first->second;
+        if (!it.second) return id;
       }
-    if (att_sets.empty()) att_sets.assign(4, make_float4(0.f, 0.f, 0.f, 0.f));
-    if (mixed) {
-      att_pset.swap(pset);
-    } else {
+      for (int l = 0; l < 3; ++l) att_sets.push_back(coef(p, l));
+      return id;
+    };
+    if (!mixed) {
       att_eset.resize(pml_slot0);
-      for (int s = 0; s < pml_slot0; ++s) att_eset[s] = pset[S->lane_index(s, 0)];
+      for (int s = 0; s < pml_slot0; ++s) att_eset[s] = set_of(first(s, 0));
+    } else {
+      att_pset.assign(nq, 0);
+      for (int s = 0; s < pml_slot0 && seen.size() <= MAX_POINT_SETS; ++s)
+        for (int q = 0; q < NGLL2; ++q) att_pset[S->lane_index(s, q)] = set_of(first(s, q));
+      if (seen.size() > MAX_POINT_SETS) {
+        att_pset.clear();
+        att_sets.clear();
+        att_coef.assign(3 * nq, make_float4(0.f, 0.f, 0.f, 0.f));
+        for (int s = 0; s < pml_slot0; ++s)
+          for (int q = 0; q < NGLL2; ++q) {
+            const size_t k = S->lane_index(s, q);
+            for (int l = 0; l < 3; ++l) att_coef[(k / 32 * 3 + l) * 32 + k % 32] = coef(first(s, q), l);
+          }
+      }
     }
+    if (att_sets.empty()) att_sets.assign(3, make_float4(0.f, 0.f, 0.f, 0.f));
   }
   std::vector<float2> rmass(d->nglob);
   for (int g = 0; g < d->nglob; ++g) {
@@ -356,6 +385,7 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     UP(att_sets, float4, att_sets);
     if (!att_eset.empty()) UP(att_eset, int, att_eset);
     if (!att_pset.empty()) UP(att_pset, int, att_pset);
+    if (!att_coef.empty()) UP(att_coef, float4, att_coef);
     S->att_bytes = lddrk ? (sizeof(float4) * 4 + sizeof(float) * 2) * nq : sizeof(float4) * 3 * nq;
     if ((rc = S->alloc(&S->att_buf, S->att_bytes))) return rc;
     SF2D_CUDA(cudaMemset(S->att_buf, 0, S->att_bytes));
@@ -491,7 +521,7 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     for (int k = 0; k < 5; ++k) sum += d->hprime[5 * m + k];
     P.hsum[m] = static_cast<float>(sum);
   }
-  S->tile_fn = pick_rows_kernel(aniso, atten, lddrk, kern);
+  S->tile_fn = pick_rows_kernel(aniso, atten, !att_coef.empty(), lddrk, kern);
   if (pml) {
     // the layer's tiles may be smaller than the others: their kernel gets its
     // own shared-memory layout (the largest layer tile's)

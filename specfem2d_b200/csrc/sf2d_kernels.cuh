@@ -137,6 +137,7 @@ struct Params {
   int max_q, max_local;
   float hconst[60];  // hprime[25], hprimewgll[25], wxgll[5], wzgll[5]
   float hsum[5];     // row sums of hprime
+  const float4 *att_coef;  // every point's own attenuation coefficients, per warp of rows [i][SLS][row]
 };
 
 constexpr int SHARED_NT = 256;

@@ -123,12 +123,14 @@ __device__ __forceinline__ void row_transposed(const Params &P, const float2 (&t
 // LDDRK ADE stage, compute_attenuation_viscoelastic.f90:36-236); returns the
 // sums of e1, e11, e13 over the SLS.  w5i: 5 x warp + i of the point, so that
 // the arrays are [warp][i][..][lane].  Coefficients: Newmark {A1, A2, B1, B2},
-// LDDRK {1/tau1, 1/tau2, phi1, phi2} per SLS, from the point's set.
-template <bool LDDRK>
+// LDDRK {1/tau1, 1/tau2, phi1, phi2} per SLS, from the point's set or its own.
+template <bool LDDRK, bool OWN>
 __device__ __forceinline__ void attenuation_point(const Params &P, size_t w5i, int lane, int set, float dux_dxl,
                                                   float dux_dzl, float duz_dxl, float duz_dzl, int stage, float &e1s,
                                                   float &e11s, float &e13s) {
-  const float4 cc[3] = {__ldg(P.att_sets + 3 * set), __ldg(P.att_sets + 3 * set + 1), __ldg(P.att_sets + 3 * set + 2)};
+  float4 cc[3];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) cc[s] = OWN ? __ldg(P.att_coef + w5i * 96 + 32 * s + lane) : __ldg(P.att_sets + 3 * set + s);
   const float theta_n = dux_dxl + duz_dzl;
   if (!LDDRK) {
     float4 *st = P.att_a + (w5i * 3) * 32 + lane;
@@ -209,7 +211,15 @@ __device__ __forceinline__ float2 kernel_point(float2 dxi, float2 dg, float2 bxi
 // from 96.
 constexpr int row_regs(bool atten, bool kern) { return atten || kern ? 96 : 80; }
 
-template <bool ANISO, bool ATTEN, bool LDDRK, bool KERN>
+// OWN: every point reads coefficients of its own, 48 bytes that a warp reads in
+// order.  Per step of 600 x 300 elements whose points draw their set at random,
+// through the sets / OWN: 155 / 159 us with 192 sets, 162 / 159 with 3,072,
+// 174 / 159 with 49,152, 192 / 159 where all points differ; 301 x 150 with LDDRK
+// 434 / 456 us with 3,072, 451 / 456 with 49,152, 472 / 456 with 390,000 (where
+// finding 49,152 sets takes 0.2 s more than a solver without).  A medium that is
+// constant inside elements stays with the sets (148 us where all elements
+// differ).
+template <bool ANISO, bool ATTEN, bool LDDRK, bool KERN, bool OWN>
 __global__ void __maxnreg__(row_regs(ATTEN, KERN))
     k_elastic_rows(const Params P, int record_prev, int stage, int tile0, int kstep) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -258,6 +268,7 @@ __global__ void __maxnreg__(row_regs(ATTEN, KERN))
   // what is read and written in place goes to L2 meanwhile
   if (lane == 0 && (tid & ~31) < 5 * ti.nelem) {
     if (ATTEN) prefetch_l2(P.att_a + wbase * 5 * (LDDRK ? 2 : 3) * 32, 5 * (LDDRK ? 2 : 3) * 32 * sizeof(float4));
+    if (OWN) prefetch_l2(P.att_coef + wbase * 5 * 96, 5 * 96 * sizeof(float4));
     if (ATTEN && LDDRK) {
       prefetch_l2(P.att_al + wbase * 5 * 2 * 32, 5 * 2 * 32 * sizeof(float4));
       prefetch_l2(P.att_c + wbase * 5 * 32, 5 * 32 * sizeof(float));
@@ -385,7 +396,7 @@ __global__ void __maxnreg__(row_regs(ATTEN, KERN))
       }
     }
     int aset = 0, arow = -1;
-    if (ATTEN && P.att_eset) aset = __ldg(P.att_eset + ti.elem_base + e);
+    if (ATTEN && !OWN && P.att_eset) aset = __ldg(P.att_eset + ti.elem_base + e);
     if (ANISO && (phase >> 31)) arow = __ldg(P.rani + ti.elem_base + e);
     float2 t1[5];
 #pragma unroll
@@ -417,9 +428,9 @@ __global__ void __maxnreg__(row_regs(ATTEN, KERN))
         sxz = static_cast<float>(c15 * dux_dxl + c35 * duz_dzl + c55 * sh);
       }
       if (ATTEN) {
-        if (P.att_pset) aset = __ldg(P.att_pset + (wbase * 5 + i) * 32 + lane);
+        if (!OWN && P.att_pset) aset = __ldg(P.att_pset + (wbase * 5 + i) * 32 + lane);
         float e1s, e11s, e13s;
-        attenuation_point<LDDRK>(P, wbase * 5 + i, lane, aset, dux_dxl, dux_dzl, duz_dxl, duz_dzl, stage, e1s, e11s, e13s);
+        attenuation_point<LDDRK, OWN>(P, wbase * 5 + i, lane, aset, dux_dxl, dux_dzl, duz_dxl, duz_dzl, stage, e1s, e11s, e13s);
         sxx = sxx + (lam + mu) * e1s + 2.f * mu * e11s;
         sxz = sxz + mu * e13s;
         szz = szz + (lam + mu) * e1s - 2.f * mu * e11s;

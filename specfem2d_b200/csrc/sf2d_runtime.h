@@ -75,17 +75,19 @@ inline int row_tile_elems(int asked, int standard, int n) {
   return te;
 }
 
-inline TileKernel pick_rows_kernel(bool aniso, bool atten, bool lddrk, bool kern) {
-  if (kern) {  // Newmark
-    if (aniso) return atten ? k_elastic_rows<true, true, false, true> : k_elastic_rows<true, false, false, true>;
-    return atten ? k_elastic_rows<false, true, false, true> : k_elastic_rows<false, false, false, true>;
-  }
+template <bool ANISO, bool ATTEN, bool OWN>
+inline TileKernel pick_rows_kernel(bool lddrk, bool kern) {
+  if (kern) return k_elastic_rows<ANISO, ATTEN, false, true, OWN>;  // Newmark
+  return lddrk ? k_elastic_rows<ANISO, ATTEN, true, false, OWN> : k_elastic_rows<ANISO, ATTEN, false, false, OWN>;
+}
+// own: every point has attenuation coefficients of its own
+inline TileKernel pick_rows_kernel(bool aniso, bool atten, bool own, bool lddrk, bool kern) {
   if (aniso) {
-    if (atten) return lddrk ? k_elastic_rows<true, true, true, false> : k_elastic_rows<true, true, false, false>;
-    return lddrk ? k_elastic_rows<true, false, true, false> : k_elastic_rows<true, false, false, false>;
+    if (!atten) return pick_rows_kernel<true, false, false>(lddrk, kern);
+    return own ? pick_rows_kernel<true, true, true>(lddrk, kern) : pick_rows_kernel<true, true, false>(lddrk, kern);
   }
-  if (atten) return lddrk ? k_elastic_rows<false, true, true, false> : k_elastic_rows<false, true, false, false>;
-  return lddrk ? k_elastic_rows<false, false, true, false> : k_elastic_rows<false, false, false, false>;
+  if (!atten) return pick_rows_kernel<false, false, false>(lddrk, kern);
+  return own ? pick_rows_kernel<false, true, true>(lddrk, kern) : pick_rows_kernel<false, true, false>(lddrk, kern);
 }
 
 // the kernel of a CPML layer's tiles (isotropic, forward); visco: some layer

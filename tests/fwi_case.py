@@ -18,12 +18,13 @@ NX, NZ, L, H = 40, 24, 4000.0, 2400.0
 
 
 class Case:
-    def __init__(self, nstep: int = 900, qmu: float | None = None):
+    def __init__(self, nstep: int = 900, qmu: float | None = None, time_scheme: int = 1):
         interfaces = [([0.0, L], [0.0, 0.0]), ([0.0, L], [H, H])]
         self.mesh = internal_mesh(0.0, L, NX, interfaces, [NZ], absorb=(True, True, False, True))
         self.x, self.z = _gll_points(self.mesh, GLL())
         self.nstep = nstep
         self.qmu = qmu
+        self.time_scheme = time_scheme
         vp0 = 3000.0 + 0.3 * (H - self.z)
         vs0 = vp0 / 1.73
         self.rho0 = 2500.0 + 0 * self.x
@@ -40,7 +41,7 @@ class Case:
         if self.qmu is not None:
             q = dict(qkappa=np.full_like(rho, 9999.0), qmu=np.full_like(rho, self.qmu))
         return build_database(self.mesh, rho, vp, vs, [src], recs, self.nstep, 1.5e-3, stacey=True,
-                              external_model=True, **q)
+                              external_model=True, time_scheme=self.time_scheme, **q)
 
     def anomaly(self, cx=2400.0, cz=1200.0, r=300.0):
         return np.exp(-((self.x - cx) ** 2 + (self.z - cz) ** 2) / r ** 2)

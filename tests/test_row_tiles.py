@@ -45,8 +45,16 @@ def turned(db, seed=0):
 
 
 def _db(physics, nstep):
-    c = Case(nstep=nstep, qmu=40.0 if physics.startswith("visco") else None)
+    c = Case(nstep=nstep, qmu=40.0 if physics.startswith("visco") else None, time_scheme=2 if "lddrk" in physics else 1)
     db = c.start_db()
+    if physics.endswith(("mixed", "point")):
+        # coefficients that differ inside the elements: two sets, which points
+        # name, or 24,000, which are more than are shared
+        f = np.arange(25).reshape(5, 5) % 2 + np.zeros(db.ibool.shape)
+        if physics.endswith("point"):
+            f = np.random.default_rng(4).uniform(0.0, 50.0, db.ibool.shape)
+        for k in ("b1", "b2", "phi1", "phi2"):
+            db.atten[k] = (db.atten[k] * (1.0 + 1e-3 * f)[..., None]).astype(np.float32)
     if physics == "aniso":
         f32 = np.float32
         k, m = db.kappastore, db.mustore
@@ -69,17 +77,14 @@ def test_row_tiles_of_a_mesh_without_orientation(tile_elems):
 @pytest.mark.gpu
 @pytest.mark.parametrize("physics,tile_elems", [("iso", 1), ("iso", 17), ("iso", 32), ("iso", 256), ("aniso", 31),
                                                 ("aniso", 128), ("visco", 16), ("visco", 48), ("visco", 128),
-                                                ("visco mixed", 32)])
+                                                ("visco mixed", 32), ("visco point", 32),
+                                                ("visco lddrk mixed", 16), ("visco lddrk point", 17)])
 def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
     import oracle
     from specfem2d_b200.runtime import ElasticSolver
 
     n = 400
     db = _db(physics, n)
-    if physics == "visco mixed":
-        # coefficients that differ inside the elements: one set per point
-        for k in ("a1", "b1", "a2", "b2"):
-            db.atten[k] = (db.atten[k] * (1.0 + 1e-3 * (np.arange(25).reshape(5, 5) % 2))[None, :, :, None]).astype(np.float32)
     s = ElasticSolver(turned(db), tile_elems=tile_elems)
     assert s.layout_info()["max_elems"] == min(tile_elems, 128)
     seis = s.run(n)
@@ -91,7 +96,7 @@ def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("physics,tile_elems", [("iso", 0), ("iso", 33), ("iso", 128), ("visco", 0), ("visco", 64),
-                                                ("visco", 128)])
+                                                ("visco", 128), ("visco point", 32)])
 def test_lane_gradient_on_a_mesh_without_orientation(physics, tile_elems):
     import oracle
     from specfem2d_b200.fwi import FWIGradient
