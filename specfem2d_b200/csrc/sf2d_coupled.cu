@@ -713,13 +713,13 @@ extern "C" int sf2d_coupled_create(const sf2d_elastic_desc *eld, const sf2d_acou
   if ((rc = C->upload(&C->d_dev2glob, T.dev2glob.data(), T.dev2glob.size()))) return rc;
   if ((rc = C->alloc(&C->d_stage, ad->nglob))) return rc;
   C->smem = ac_row_smem_layout(A.max_local_l, A.max_elems_l, adjoint).total;
-  if (C->smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "fluid tile too large for shared memory");
+  if (C->smem > MAX_TILE_SMEM) return fail(SF2D_ERR_INVALID, "fluid tile too large for shared memory");
   C->tile_fn = adjoint ? k_acoustic_rows<false, true>
                        : C->lddrk ? k_acoustic_rows<true, false> : k_acoustic_rows<false, false>;
   if (pml_ac) {
     C->pml_fn = pick_ac_pml_tile(C->nt, C->lddrk);
     C->pml_smem = ac_smem_layout(A.max_q, A.max_local).total;
-    if (C->pml_smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "fluid tile too large for shared memory");
+    if (C->pml_smem > MAX_TILE_SMEM) return fail(SF2D_ERR_INVALID, "fluid tile too large for shared memory");
     if (C->pml_tile0 > 0 && C->pml_tile0 < T.ntiles) {
       SF2D_CUDA(cudaStreamCreateWithPriority(&C->side, cudaStreamNonBlocking, C->el ? C->el->priority : 0));
       SF2D_CUDA(cudaEventCreateWithFlags(&C->ev_fork, cudaEventDisableTiming));

@@ -109,12 +109,22 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   auto *S = new sf2d_solver();
   std::unique_ptr<sf2d_solver> guard(S);
   if (d->tile_elems > 256) return fail(SF2D_ERR_INVALID, "tiling: tile_elems must be in [1, 256]");
-  const int te = row_tile_elems(d->tile_elems, 64, d->nspec);
-  const int group_te[3] = {te, te, d->pml_tile_elems > 0 ? d->pml_tile_elems : tile_hint(d->tile_elems, 64)};
-  std::string err = build_tiling(d->nspec, d->nglob, d->ibool, d->centroid_xz, te, S->T,
-                                 grouped ? group.data() : nullptr, grouped ? 3 : 1, grouped ? group_te : nullptr,
-                                 grouped ? 2 : 1);
-  if (!err.empty()) return fail(SF2D_ERR_INVALID, "tiling: " + err);
+  int te = row_tile_elems(d->tile_elems, 64, d->nspec);
+  const int pml_te = d->pml_tile_elems > 0 ? d->pml_tile_elems : tile_hint(d->tile_elems, 64);
+  std::string err;
+  for (;; te /= 2) {
+    const int group_te[3] = {te, te, pml_te};
+    err = build_tiling(d->nspec, d->nglob, d->ibool, d->centroid_xz, te, S->T, grouped ? group.data() : nullptr,
+                       grouped ? 3 : 1, grouped ? group_te : nullptr, grouped ? 2 : 1);
+    if (!err.empty()) return fail(SF2D_ERR_INVALID, "tiling: " + err);
+    // Scattered elements (a numbering without order and no centres) hold up to
+    // 25 points each, which 128 of an adjoint run have no room for.  Its forward
+    // run has the same tiles: its frames are in their numbering.
+    int nl = 0;
+    for (int t = 0; t < (grouped ? S->T.group_tile_begin[2] : S->T.ntiles); ++t)
+      nl = std::max(nl, S->T.tiles[t].n_int + S->T.tiles[t].n_sh);
+    if (row_smem_layout(nl, te, true).total <= MAX_TILE_SMEM || te == 1) break;
+  }
   const Tiling &T = S->T;
   S->late_tile0 = late_elem ? T.group_tile_begin[1] : 0;
   for (int k = 0; k < d->nsrc; ++k)
@@ -504,7 +514,7 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     P.hconst[55 + k] = d->wzgll[k];
   }
   S->smem = row_smem_layout(P.max_local, P.max_elems, kern).total;
-  if (S->smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "tile too large for shared memory");
+  if (S->smem > MAX_TILE_SMEM) return fail(SF2D_ERR_INVALID, "tile too large for shared memory");
   S->nt = d->threads_per_block > 0 ? d->threads_per_block : 256;
   if (S->nt != 128 && S->nt != 250 && S->nt != 256 && S->nt != 512)
     return fail(SF2D_ERR_INVALID, "threads_per_block must be 128, 250, 256 or 512");
@@ -534,7 +544,7 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
     S->pml_max_local = pl;
     S->pml_fn = pick_pml_kernel(S->pml_nt, lddrk, pml_visco);
     S->pml_smem = tile_smem_layout(S->pml_max_q, S->pml_max_local).total;
-    if (S->pml_smem > 220 * 1024) return fail(SF2D_ERR_INVALID, "tile too large for shared memory");
+    if (S->pml_smem > MAX_TILE_SMEM) return fail(SF2D_ERR_INVALID, "tile too large for shared memory");
   }
   S->lddrk = lddrk;
   S->nstage = nstage;

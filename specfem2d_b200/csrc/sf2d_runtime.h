@@ -55,6 +55,7 @@ using TileKernel = void (*)(Params, int, int, int, int);
 // Five threads an element and at most 96 registers a thread: 128 elements fit
 // a CTA and the register file.
 constexpr int MAX_ROW_ELEMS = 128;
+constexpr size_t MAX_TILE_SMEM = 220 * 1024;
 
 // A description's tile_elems: > 0 as given; -n "up to n"; 0 up to `standard`.
 inline int tile_hint(int asked, int standard) {

@@ -116,3 +116,44 @@ def test_lane_gradient_on_a_mesh_without_orientation(physics, tile_elems):
         got = np.array(got)
         got[flip] = got[flip][:, ::-1, ::-1]
         assert rel_l2(got, r64) < max(1e-5, 1.5 * rel_l2(r32, r64))
+
+
+@pytest.mark.gpu
+def test_gradient_on_tiles_of_scattered_elements(monkeypatch):
+    """Elements in random order and no element centres: a tile of 128 holds more
+    than 3,064 points, more than an adjoint run has shared memory for, so both
+    runs take smaller tiles.  Against the ordered mesh, whose sums are in
+    another order (1e-4, four times what that changes in a kernel)."""
+    from specfem2d_b200 import configs, fwi, runtime
+
+    n = 500
+    db = configs.c1_homogeneous(nstep=n)
+    perm = np.random.default_rng(1).permutation(db.nspec)
+    mixed = copy.copy(db)
+    for k in ("ibool", "xix", "xiz", "gammax", "gammaz", "jacobian", "rhostore", "kappastore", "mustore", "rho_vpstore",
+              "rho_vsstore"):
+        setattr(mixed, k, np.ascontiguousarray(getattr(db, k)[perm]))
+    new = np.argsort(perm).astype(np.int32)
+    mixed.source_ispec, mixed.rec_ispec = new[db.source_ispec], new[db.rec_ispec]
+    shared = [mixed.ibool[k:k + 128].reshape(-1) for k in range(0, db.nspec, 128)]
+    assert max(len(np.unique(p)) for p in shared) > 3064
+    t = np.arange(n)[None, :, None] / n
+    adj = np.sin(2 * np.pi * np.random.default_rng(2).uniform(2, 6, (len(db.rec_ispec), 1, 2)) * t) * np.sin(np.pi * t) ** 2
+
+    def kernels(d, **kw):
+        g = fwi.FWIGradient(d, 125, **kw)
+        seis = g.forward()
+        return [seis] + list(g.backward(adj))
+
+    ref = kernels(db)
+
+    def without_centres(*a):
+        d, keep = runtime.build_desc(*a)
+        d.centroid_xz = None
+        return d, keep
+
+    monkeypatch.setattr(fwi, "build_desc", without_centres)
+    got = kernels(mixed, tile_elems=128)
+    assert rel_l2(got[0], ref[0]) < 1e-5
+    for a, b in zip(got[1:], ref[1:]):
+        assert np.linalg.norm(b) > 0 and rel_l2(a, b[perm]) < 1e-4
