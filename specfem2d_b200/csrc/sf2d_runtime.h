@@ -63,6 +63,13 @@ inline int tile_hint(int asked, int standard) {
   return asked > 0 ? asked : standard;
 }
 
+inline int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 148;
+  return n;
+}
+
 // Elements per tile by rows of a mesh (or domain) of n elements.  A size that
 // is asked for is used; "up to" is halved (to 8 at least) while the tiles would
 // not give every SM one and every other SM a second.  A step of a small mesh
@@ -72,7 +79,8 @@ inline int tile_hint(int asked, int standard) {
 inline int row_tile_elems(int asked, int standard, int n) {
   int te = std::min(tile_hint(asked, standard), MAX_ROW_ELEMS);
   if (asked > 0) return te;
-  while (te >= 16 && 2 * static_cast<long long>((n + te - 1) / te) < 3 * 148) te /= 2;
+  const long long sms = sm_count();
+  while (te >= 16 && 2 * static_cast<long long>((n + te - 1) / te) < 3 * sms) te /= 2;
   return te;
 }
 
