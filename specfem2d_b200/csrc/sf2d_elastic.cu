@@ -521,11 +521,6 @@ int sf2d_create_solver_internal(const sf2d_elastic_desc *d, bool kern, sf2d_solv
   S->pml_nt = d->pml_threads_per_block > 0 ? d->pml_threads_per_block : S->nt;
   if (S->pml_nt != 128 && S->pml_nt != 250 && S->pml_nt != 256 && S->pml_nt != 512)
     return fail(SF2D_ERR_INVALID, "pml_threads_per_block must be 128, 250, 256 or 512");
-  if (d->nrec > 0) {
-    for (int t = S->pml_tile0; t < T.ntiles; ++t)
-      if (tiles[t].rec_n > S->pml_nt)
-        return fail(SF2D_ERR_INVALID, "more receivers in one tile than threads per CTA");
-  }
   for (int m = 0; m < 5; ++m) {
     double sum = 0.0;
     for (int k = 0; k < 5; ++k) sum += d->hprime[5 * m + k];

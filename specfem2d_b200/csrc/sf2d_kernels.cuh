@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(NT, 768 / NT)
 
   const int step = *P.d_step + kstep;
   // receivers of the previous step read the old fields before any write
-  if (record_prev && tid < ti.rec_n) record_receiver(P, ti.rec_off + tid, step - 1);
+  if (record_prev)
+    for (int r = tid; r < ti.rec_n; r += NT) record_receiver(P, ti.rec_off + r, step - 1);
   // a masked member neither reads nor writes its points from here on (uniform over the CTA)
   if (P.tile_member && P.member_status[P.tile_member[tile0 + blockIdx.x]]) return;
 

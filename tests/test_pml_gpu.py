@@ -238,3 +238,25 @@ def test_coupled_cpml_chunking_is_bitwise(c2_pml):
     fa, fb = a.get_fields(), b.get_fields()
     for k in ("displ", "veloc", "pot", "pot_dot"):
         assert np.array_equal(fa[k], fb[k])
+
+
+def test_more_receivers_in_a_layer_tile_than_threads():
+    """How many receivers one element of a layer may hold does not depend on the
+    tile it falls into: 600 copies of a receiver record its trace."""
+    import copy
+
+    from specfem2d_b200.runtime import ElasticSolver
+
+    cfg, _ = load_golden("semi_infinite_homogeneous")
+    db = database_from_config(cfg)
+    e = int(np.flatnonzero(np.asarray(db.pml["region"]) > 0)[100])
+
+    def run(n):
+        d = copy.copy(db)
+        d.rec_ispec = np.full(n, e, dtype=np.int32)
+        d.hxir, d.hgammar = np.repeat(db.hxir[:1], n, 0), np.repeat(db.hgammar[:1], n, 0)
+        return ElasticSolver(d, pml_threads_per_block=128).run(300)
+
+    one, many = run(1), run(600)
+    assert many.shape[0] == 600 and np.abs(one).max() > 0
+    assert np.array_equal(many, np.repeat(one, 600, 0))
