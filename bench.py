@@ -83,13 +83,11 @@ def build_workload(name: str, nstep: int, rank: int = 0, dist=None, scale: int =
 # steps of the configuration's whole run (the end-to-end leg over the full run)
 WORKLOAD_NSTEP = {"c1": 2000, "c2_coupled": 6000, "c3_viscoelastic": 8000}
 
-
-# DRAM bytes one step's solid tile launches move (read + write), measured with
-# ncu on one B200 for the workload and tile configuration of the key
-# (workload, tile elements, threads, fluid tile elements, CPML tile elements,
-# CPML threads); the roofline's "traffic" reports it beside the algorithmic bytes
-TILE_TRAFFIC = {}  # none taken yet with the kernels by element rows
-TRAFFIC_SOURCE = {}
+# DRAM bytes (read, written) of one launch of the solid's tile kernel, measured
+# with ncu on one B200 at full size, per workload and elements per tile; the
+# roofline's "traffic" reports their sum beside the algorithmic bytes
+TILE_TRAFFIC = {("c3_viscoelastic", 32): (3085.5e6, 1957.3e6)}
+TRAFFIC_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum of one tile launch at full size"
 
 WORKLOAD_DESC = {
     "c2_coupled": ("800x320-element (20 km x 8 km, 4,100,481 GLL points) coupled fluid-solid model: 1 km "
@@ -446,7 +444,7 @@ def run_fwi(args, rank, world):
                    "nspec_total": sum(m.nspec for m in all_models), "nglob_total": r["nglob_total"],
                    "checkpoint_every": r["checkpoint_every"],
                    "parallelism": f"models sharded over {world} GPU(s)",
-                   "tile_elems": args.tile_elems, "threads_per_cta": args.threads},
+                   "tile_elems": args.tile_elems or "by mesh size (up to 32)"},
         **{k: r[k] for k in ("plain_s_per_shot", "batched_s_per_shot", "speedup_batched_vs_plain",
                              "gradient_rel_l2_batched_vs_plain", "point_updates_per_s_batched",
                              "summed_gradient")},
@@ -468,7 +466,7 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
     import torch
 
     from specfem2d_b200.configs import (algorithmic_bytes_coupled, algorithmic_bytes_elastic,
-                                        algorithmic_bytes_viscoelastic)
+                                        algorithmic_bytes_viscoelastic, tile_launch_bytes)
     from specfem2d_b200.coupled import CoupledSolver
     from specfem2d_b200.distributed import job_throughput, max_over_ranks
     from specfem2d_b200.runtime import ElasticSolver
@@ -482,7 +480,7 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
             (args.fluid_tile_elems, args.pml_tile_elems, args.pml_threads), tune = autotune_coupled(
                 db, args.tile_elems, args.threads)
         else:
-            (args.tile_elems, args.threads), tune = autotune_elastic(db, tiles=(32, 48, 64), threads=(256, 512),
+            (args.tile_elems, args.threads), tune = autotune_elastic(db, tiles=(0, 32, 48, 64), threads=(256, 512),
                                                                      steps=10, warmup=3)
 
     def make_solver():
@@ -530,29 +528,18 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
     st = solver.solid_layout_info() if coupled else solver.layout_info()
     nsh = st["nshared"]
     n_int = el_db.nglob - nsh
-    # algorithmic bytes of the (solid) element kernel per launch: element data + interior points
-    # (u, v, a read+write, rmass) + shared points touched by tiles (u, v, a read, partial write)
     n_slots = st["n_slots"]
     pm = getattr(db, "pml", None)
     npml_el = int((el_db.pml["region"] > 0).sum()) if getattr(el_db, "pml", None) is not None else 0
     npml_ac = int((pm["region"] > 0).sum()) - npml_el if pm is not None else 0
+    tile_bytes = tile_launch_bytes(el_db.nspec, n_int, n_slots, el_db.atten is not None, int(db.time_scheme), npml_el)
     if db.atten is None:
-        # + per CPML element point: damping profiles (48 B), rho J (4 B), memory variables read + write (96 B)
-        tile_bytes = 700 * el_db.nspec + 56 * n_int + 32 * n_slots + 25 * 148 * npml_el
         step_bytes = algorithmic_bytes_elastic(db.nspec, db.nglob)
-    elif db.time_scheme == 1:
-        tile_bytes = 700 * db.nspec + 3600 * db.nspec + 56 * n_int + 32 * n_slots
-        step_bytes = algorithmic_bytes_viscoelastic(db.nspec, db.nglob, 1)
     else:
-        # per stage: element data, memory variables and their LDDRK copies, coefficients,
-        # interior points (u, v, u_L, v_L read+write, a written, rmass read), shared reads + partial
-        tile_bytes = db.nspec * (700 + 25 * 192) + 88 * n_int + 24 * n_slots
-        step_bytes = algorithmic_bytes_viscoelastic(db.nspec, db.nglob, 2)
+        step_bytes = algorithmic_bytes_viscoelastic(db.nspec, db.nglob, int(db.time_scheme))
     if coupled:
         step_bytes = algorithmic_bytes_coupled(el_db.nspec, el_db.nglob, solver.nspec_fluid, solver.nglob_fluid,
                                                npml_el, npml_ac)
-    traffic_key = (workload, args.tile_elems, args.threads, args.fluid_tile_elems, args.pml_tile_elems,
-                   args.pml_threads)
     peaks = {}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -561,6 +548,7 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
         pass
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = tile_bytes / (tile_ms * 1e-3) / 1e9
+    traffic = TILE_TRAFFIC.get((workload, st["max_elems"])) if args.scale == 1 else None
     solver.close()
 
     def pinned(shape, dtype):
@@ -616,12 +604,12 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
     return {
         "value": value, "ms_per_step": ms / K,
         "config": {"workload": workload, "description": WORKLOAD_DESC[workload], "scale": args.scale,
-                   "nspec": db.nspec, "nglob": db.nglob, "tile_elems": args.tile_elems,
+                   "nspec": db.nspec, "nglob": db.nglob, "tile_elems": st["max_elems"],
+                   "threads_per_cta": st["threads_per_block"],
                    "fluid_tile_elems": (args.fluid_tile_elems or args.tile_elems) if coupled else None,
-                   "fluid_threads_per_cta": (args.fluid_threads or args.threads) if coupled else None,
-                   "cpml_tile_elems": args.pml_tile_elems or args.tile_elems,
-                   "cpml_threads_per_cta": args.pml_threads or args.threads,
-                   "threads_per_cta": args.threads, "autotuned": bool(tune),
+                   "cpml_tile_elems": (args.pml_tile_elems or args.tile_elems) if npml_el else None,
+                   "cpml_threads_per_cta": (args.pml_threads or args.threads) if npml_el else None,
+                   "autotuned": bool(tune),
                    "autotune_candidates": tune,
                    "ntiles": st["ntiles"], "shared_points": nsh,
                    "nspec_fluid": solver.nspec_fluid if coupled else 0,
@@ -636,8 +624,8 @@ def measure_forward(db, args, workload, K, W, world, dist, nstep_full=0):
         "local_point_updates_per_s": 25 * db.nspec * K * world / (ms * 1e-3),
         "s_per_element_step": ms * 1e-3 / K / db.nspec,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": TILE_TRAFFIC.get(traffic_key),
-                     "traffic_source": TRAFFIC_SOURCE.get(traffic_key),
+                     "frac": achieved / peak, "traffic": sum(traffic) if traffic else None,
+                     "traffic_source": TRAFFIC_SOURCE if traffic else None,
                      "kernel": "k_elastic_rows", "kernel_ms": tile_ms, "shared_kernel_ms": shared_ms,
                      "fluid_kernels_ms": k_ms[:2] if coupled else None, "step_kernels_ms": k_ms[-1],
                      "algorithmic_bytes_per_launch": tile_bytes,
@@ -672,10 +660,10 @@ def main():
     ap.add_argument("--fwi-set", default="first", choices=["first", "smallest"],
                     help="the first --models of the 48 seeded sizes, or the smallest")
     ap.add_argument("--batch", type=int, default=0, help="members per packed mesh in the FWI workloads (0 = all)")
-    ap.add_argument("--tile-elems", type=int, default=32)
-    ap.add_argument("--threads", type=int, default=256)
+    ap.add_argument("--tile-elems", type=int, default=0, help="solid tiles; 0 = by the mesh's size (up to 32)")
+    ap.add_argument("--threads", type=int, default=256, help="CPML CTA threads")
     ap.add_argument("--fluid-tile-elems", type=int, default=64, help="fluid tiles (coupled runs); 0 = --tile-elems")
-    ap.add_argument("--fluid-threads", type=int, default=0, help="fluid CTA threads; 0 = --threads")
+    ap.add_argument("--fluid-threads", type=int, default=0, help="fluid CPML CTA threads; 0 = --threads")
     ap.add_argument("--pml-tile-elems", type=int, default=16, help="solid CPML tiles; 0 = --tile-elems")
     ap.add_argument("--pml-threads", type=int, default=128, help="solid CPML CTA threads; 0 = --threads")
     ap.add_argument("--no-autotune", dest="autotune", action="store_false",

@@ -265,13 +265,32 @@ def c3_viscoelastic(nstep: int = 8000, time_scheme: int = 1, scale: int = 1, nre
 
 
 def algorithmic_bytes_viscoelastic(nspec: int, nglob: int, time_scheme: int = 1) -> int:
-    """Bytes of one viscoelastic 3-SLS step in the reference layout: the elastic
-    step plus, per element GLL point, e1 e11 e13 (3 SLS) read + write (72 B),
-    the A/B coefficients (48 B) and the three previous strains read + write
-    (24 B) for Newmark; LDDRK does 6 stages, each with the element data, the
-    memory variables and their LDDRK copies read + write (144 B), 1/tau and
-    phi (48 B) per element point and u, v, u_L, v_L read + write, a written
-    and rmass read per global point (88 B)."""
+    """Bytes of one viscoelastic 3-SLS step: the elastic step plus, per element
+    GLL point, e1 e11 e13 (3 SLS) and the three previous strains read + write
+    (96 B) for Newmark; LDDRK does 6 stages, each with the element data, the
+    memory variables and their LDDRK copies read + write (144 B) per element
+    point and u, v, u_L, v_L read + write, a written and rmass read per global
+    point (88 B).  The coefficients of the relaxation are equal for whole media
+    and count as the 4 B that name an element's set, not as the 48 B per point
+    of the reference's layout."""
     if time_scheme == 1:
-        return 700 * nspec + 56 * nglob + 3600 * nspec
-    return 6 * (nspec * (700 + 25 * 192) + nglob * 88)
+        return 700 * nspec + 56 * nglob + (25 * 96 + 4) * nspec
+    return 6 * (nspec * (700 + 25 * 144 + 4) + nglob * 88)
+
+
+def tile_launch_bytes(nspec: int, n_int: int, n_slots: int, atten: bool = False, time_scheme: int = 1,
+                      npml: int = 0) -> int:
+    """Bytes the tile kernels of one step (LDDRK: one stage) have to move, in the
+    layout they use.  Per element: mapping and moduli of 25 points (24 B each),
+    the local ids of five rows (12 B each), the assembly phases (4 B); with 3 SLS
+    the memory variables and previous strains of 25 points read and written
+    (2 x 48 B; LDDRK 2 x 72 B) and the element's coefficient set (4 B); per CPML
+    element damping profiles (48 B), rho J (4 B) and memory variables read and
+    written (96 B) of 25 points.  Per interior point: u, v, a read and written and
+    the inverse mass read (56 B; LDDRK u, v, u_L, v_L read and written, a written:
+    88 B); per partial-sum slot the same fields read and the sum written."""
+    per_elem = 25 * 24 + 5 * 12 + 4
+    if atten:
+        per_elem += 25 * (96 if time_scheme == 1 else 144) + 4
+    points = 56 * n_int + 32 * n_slots if time_scheme == 1 else 88 * n_int + 24 * n_slots
+    return per_elem * nspec + points + 25 * 148 * npml
