@@ -75,10 +75,12 @@ inline int sm_count() {
 // not give every SM one and every other SM a second.  A step of a small mesh
 // takes as long as one tile does: 80 x 60 elements take 9.9 us with 150 tiles of
 // 32 and 8.8 us with 300 of 16; 233 x 147 elements (1071 tiles of 32) 17.9 us,
-// and 19.1 us in tiles of 16.
+// and 19.1 us in tiles of 16.  Up to 32 elements stay in one tile, which needs no
+// kernel for shared points: 3 x 3 elements 7.8 us, and 9.0 in tiles of 8; 6 x 5
+// 7.8 and 8.9; 8 x 8 8.8 and 8.3.
 inline int row_tile_elems(int asked, int standard, int n) {
   int te = std::min(tile_hint(asked, standard), MAX_ROW_ELEMS);
-  if (asked > 0) return te;
+  if (asked > 0 || n <= std::min(te, 32)) return te;
   const long long sms = sm_count();
   while (te >= 16 && 2 * static_cast<long long>((n + te - 1) / te) < 3 * sms) te /= 2;
   return te;

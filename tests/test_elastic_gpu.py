@@ -161,6 +161,27 @@ def test_tile_size_is_the_callers_and_otherwise_fits_the_mesh(tromp):
     assert ElasticSolver(db).layout_info()["max_elems"] == 8
 
 
+@pytest.mark.parametrize("nx,nz,ntiles", [(1, 1, 1), (3, 3, 1), (8, 4, 1), (11, 3, 5)])
+def test_few_elements_stay_in_one_tile(nx, nz, ntiles):
+    """Up to 32 elements by default: one tile, one kernel a step, and the traces
+    of tiles of 8."""
+    from specfem2d_b200.runtime import ElasticSolver
+    from specfem2d_b200.setup.mesh import internal_mesh
+    from specfem2d_b200.setup.solver_setup import Source, build_database
+
+    x, z = 100.0 * nx, 100.0 * nz
+    mesh = internal_mesh(0.0, x, nx, [([0.0, x], [0.0, 0.0]), ([0.0, x], [z, z])], [nz], absorb=(True, True, False, True))
+    one = np.ones((nx * nz, 5, 5))
+    db = build_database(mesh, 2000.0 * one, 3000.0 * one, 1700.0 * one, [Source(x=0.4 * x, z=0.6 * z, f0=8.0, factor=1e10)],
+                        [(0.7 * x, z)], 200, 1.5e-3, stacey=True, external_model=True)
+    s = ElasticSolver(db)
+    assert s.layout_info()["ntiles"] == ntiles
+    if ntiles == 1:
+        assert s.launch_count(1) == 2  # the tile, the step counter
+    a, b = s.run(200), ElasticSolver(db, tile_elems=8).run(200)
+    assert np.abs(b).max() > 0 and rel_l2(a, b) < TOL
+
+
 def test_initialize_device_selects_rank_modulo_devices(tromp):
     """sf2d_initialize_device (initialize_cuda_device): rank % visible devices
     becomes current in the library's runtime, and a solver created afterwards
