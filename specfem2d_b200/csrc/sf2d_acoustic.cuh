@@ -1,13 +1,14 @@
-// Device side of the tile-staged acoustic (fluid) time step, NGLL = 5.
+// Device side of the tile-staged acoustic (fluid) time step, NGLL = 5: what its
+// kernels share, the kernel of the CPML tiles and the one that finishes shared
+// points.  The other tiles' kernel is in sf2d_acoustic_rows.cuh.
 //
 // The fluid is solved for the scalar potential chi with u = grad(chi) / rho
 // and pressure p = -chi_dot_dot (compute_forces_viscoacoustic.f90:34-417).
 // It uses the same tiling as the solid (sf2d_tiler.h) over the fluid
 // elements, with its own device numbering of the fluid points.  One CTA per
 // tile and time step (or LDDRK stage):
-//   1. cp.async of local ibool and chi, chi_dot, chi_dot_dot of the tile's
-//      points into shared memory (geometry and J/rho are read from global
-//      memory where they are used);
+//   1. cp.async of chi, chi_dot, chi_dot_dot of the tile's points (and a CPML
+//      tile's local ibool) into shared memory;
 //   2. Newmark predictor (update_displacement_Newmark.F90:353-402) or a
 //      cleared accumulator (LDDRK), free-surface points zeroed
 //      (enforce_acoustic_free_surface.f90:35-96);
@@ -17,11 +18,11 @@
 //      chi_dd += w (u . n) (compute_coupling_acoustic_el.f90:60-283, with the
 //      solid's predicted displacement formed here from its u, v, a), the
 //      pressure sources chi_dd += s stf / kappa (compute_add_sources_acoustic.f90:49-75);
-//   4. derivative lines through hprime (one thread per element row or
-//      column), per GLL point the mapping and J/rho weak-form terms
-//      (compute_forces_viscoacoustic.f90:105-238), weighted transpose lines
-//      with hprimewgll (:306-322);
-//   5. assembly colour by colour;
+//   4. derivatives through hprime, per GLL point the mapping and J/rho weak-form
+//      terms (compute_forces_viscoacoustic.f90:105-238), weighted transposes
+//      with hprimewgll (:306-322); CPML tiles by lines (one thread per element
+//      row or column) and points, with the layer's memory variables;
+//   5. assembly phase by phase, in CPML tiles colour by colour;
 //   6. interior points: chi_dd *= rmass_inverse, corrector or LDDRK update
 //      (update_displacement_Newmark.F90:631-662, update_displacement_LDDRK.F90:88-115),
 //      free-surface zeroing, write-back; shared points: partial sums.
@@ -45,7 +46,7 @@ struct AcParams {
   const float *rmass;         // rmass_inverse_acoustic
   const uint8_t *free_mask;   // 1 on free-surface points
   const TileInfo *tiles;
-  // tiles by rows (sf2d_acoustic_lanes.cuh), per block of 32 elements, arrays are [block][q][lane]
+  // tiles by rows (sf2d_acoustic_rows.cuh), per warp of 32 rows [i][row]
   const float4 *lgeo;         // xix, xiz, gammax, gammaz
   const float *lfac;          // jacobian / rho formed in FP32
   size_t nlane_q;             // their size
@@ -109,7 +110,7 @@ struct AcParams {
   const int *pframe_base;
   int npframes;
   // adjoint sweep with kernel accumulation: forward chi frame = *kp_base - step;
-  // the sums of grad(chi_adj) . grad(chi) per element point ([block][q][lane]) and of
+  // the sums of grad(chi_adj) . grad(chi) per element point ([warp][i][row]) and of
   // chi_adj_dd chi per fluid point
   const float *kpframes;
   const int *kp_base;

@@ -293,7 +293,7 @@ __global__ void __maxnreg__(AC_ROW_REGS) k_acoustic_rows(const AcParams A, int s
 }
 
 // Fluid kernel sums to element order: rho' = dt / rho sum, kappa' = dt / kappa
-// sum (one thread per element point; lane: first lane of each element).
+// sum (one thread per element point; lane: first row of each element).
 static __global__ void k_fluid_kernels(const float *kl, const float *kap_glob, const int *lane, const int *point,
                                        const float2 *rk, float dt, int n, float *out) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;

@@ -94,7 +94,7 @@ struct sf2d_coupled {
   size_t pml_smem = 0;
   size_t smem = 0;
   int lane_nt = 32;             // threads per CTA of the tiles by rows
-  std::vector<int> slot_lane;   // tiles by rows: slot -> the element's lane
+  std::vector<int> slot_lane;   // tiles by rows: slot -> the element's first row
   int nt = 256, nstage = 1, nglob = 0, nrec_total = 0, nstep = 0, steps_done = 0;
   size_t npml_q = 0;  // GLL points of the fluid CPML elements
   bool lddrk = false;

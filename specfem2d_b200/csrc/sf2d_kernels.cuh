@@ -1,7 +1,9 @@
-// Device side of the tile-staged elastic time step (NGLL = 5).
+// Device side of the tile-staged elastic time step (NGLL = 5): the parameters
+// and helpers of its kernels, the kernel of the CPML tiles and the one that
+// finishes shared points.  The other tiles' kernel is in sf2d_rows.cuh.
 //
 // One CTA advances one tile of elements by one Newmark step or one LDDRK
-// stage:
+// stage; a CPML tile's in tasks of lines, columns and points:
 //   1. cp.async of the tile's local ibool and the fields of all its points
 //      straight into shared memory (geometry and material are read from
 //      global memory where they are used);
@@ -14,12 +16,9 @@
 //      compute_add_sources_viscoelastic.f90:36-101);
 //   4. derivative lines (one thread per element row or column: the 5x5
 //      contraction with hprime, mxm_4comp_singleA :810-883), then per GLL
-//      point the Jacobian mapping, isotropic (lambda, mu as
-//      compute_forces_viscoelastic.F90:286-294 forms them) or anisotropic
-//      stress (:372-445, in double as the reference), 3-SLS memory variables
-//      and their stress correction (compute_attenuation_viscoelastic.f90:36-236,
-//      :481-503), weak-form terms (:669-675), then the weighted transpose
-//      lines with hprimewgll (:760-782);
+//      point the Jacobian mapping, the layer's memory variables, stress and
+//      acceleration terms, weak-form terms (:669-675), then the weighted
+//      transpose lines with hprimewgll (:760-782);
 //   5. assembly into the shared accumulator colour by colour (no two elements
 //      of a colour share a point: no atomics);
 //   6. interior points: a *= rmass_inverse, then the Newmark corrector

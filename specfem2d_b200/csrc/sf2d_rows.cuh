@@ -10,13 +10,13 @@
 // whole element in one or two threads' registers needs fewer operations, but
 // leaves too few warps in flight and is slower on every mesh but the largest.
 //
-// What bounds it: latency at 20 to 25 warps per SM (issue slots half used, DRAM
-// at 3.1 of 6.65 TB/s on 210,000 elements).  So all that does not change from
-// step to step is requested before the previous kernel is waited for: the
-// element data, the largest part of the bytes, into registers, the inverse mass
-// and the lists of shared points by cp.async (waiting for them in the point
-// loops cost about 1000 cycles each), and what is read and written in place
-// into L2.
+// What bounds it: latency at 19 warps per SM (1000 x 400 elements: issue slots
+// half used, DRAM at 3.6 of 6.55 TB/s); with attenuation on large meshes DRAM
+// (1600 x 800 elements: 5.0 GB in 0.855 ms, 5.9 TB/s).  So all that does not
+// change from step to step is requested before the previous kernel is waited
+// for: the element data, the largest part of the bytes, into registers, the
+// inverse mass and the lists of shared points by cp.async, and what is read and
+// written in place into L2.
 //
 // Per step, against tasks of rows, columns and points (tiles of 32 elements):
 // 80 x 60 elements 10.9 -> 9.9 us, 233 x 147 with topography 21.4 -> 17.9 us,
@@ -122,7 +122,7 @@ __device__ __forceinline__ void row_transposed(const Params &P, const float2 (&t
 // Memory-variable update of one element point (Newmark recursive convolution or
 // LDDRK ADE stage, compute_attenuation_viscoelastic.f90:36-236); returns the
 // sums of e1, e11, e13 over the SLS.  w5i: 5 x warp + i of the point, so that
-// the arrays are [warp][i][..][lane].  Coefficients: Newmark {A1, A2, B1, B2},
+// the arrays are [warp][i][..][row].  Coefficients: Newmark {A1, A2, B1, B2},
 // LDDRK {1/tau1, 1/tau2, phi1, phi2} per SLS, from the point's set or its own.
 template <bool LDDRK, bool OWN>
 __device__ __forceinline__ void attenuation_point(const Params &P, size_t w5i, int lane, int set, float dux_dxl,
@@ -247,7 +247,7 @@ __global__ void __maxnreg__(row_regs(ATTEN, KERN))
   }
   cp_async_commit();
   // what does not change from step to step is requested before the previous
-  // kernel is waited for; idle threads of the last warp read its padding
+  // kernel is waited for
   const size_t wbase = static_cast<size_t>((ti.lane0 + tid) >> 5);
   float4 geo[5];
   float2 mat[5];

@@ -252,15 +252,15 @@ struct sf2d_solver {
     Q.max_local = pml_max_local;
     return Q;
   }
-  // Tiles [first, ntiles): the plain ones on the solver stream, the CPML ones
-  // beside them on the side stream when there is one.  first = late_tile0
-  // leaves the early tiles to launch_early.
   template <typename F, typename... A>
   void launch_pdl(F fn, int grid, int block, size_t smem_bytes, A... args) {
     sf2d::launch_pdl(stream, launch_error, fn, grid, block, smem_bytes, args...);
   }
   cudaError_t launch_error = cudaSuccess;
-  // kstep: steps since the counter on the device was last advanced
+  // Tiles [first, ntiles): the plain ones on the solver stream, the CPML ones
+  // beside them on the side stream when there is one.  first = late_tile0
+  // leaves the early tiles to launch_early.
+  // kstep: steps since the counter on the device was last advanced.
   void launch_tile(bool record_prev, int stage, int first, int kstep) {
     const int rp = record_prev ? 1 : 0;
     const int nplain = pml_tile0 - first;
