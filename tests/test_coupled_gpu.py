@@ -116,3 +116,25 @@ def test_restart_and_chunking_bitwise(c2_small):
     g = s2.get_fields()
     for k in f:
         assert np.array_equal(f[k], g[k]), k
+
+
+@pytest.mark.parametrize("scheme", [1, 2])
+def test_tile_sizes_of_both_domains(c2_small, scheme):
+    """Solid and fluid tiles from one element to the largest a CTA takes."""
+    import oracle
+    from specfem2d_b200.coupled import CoupledSolver
+
+    n = 900 if scheme == 1 else 600  # the pressure has reached the receivers
+    db = c2_small if scheme == 1 else configs.c2_coupled(nstep=n, nrec=12, scale=8, time_scheme=2)
+    o32, o64 = oracle.Oracle(db, 4), oracle.Oracle(db, 8)
+    ref, ref64 = o32.run(n), o64.run(n)
+    assert np.abs(ref).max() > 0
+    nfluid = int(np.asarray(db.acoustic["ispec"]).sum())
+    for te, fte in ((1, 1), (7, 33), (64, 17), (128, 128)):
+        s = CoupledSolver(db, tile_elems=te, fluid_tile_elems=fte)
+        assert s.solid_layout_info()["max_elems"] == te and s.layout_info()["ntiles"] == -(-nfluid // fte)
+        assert _close(s.run(n), ref, ref64), (te, fte)
+        f = s.get_fields()
+        assert _close(f["displ"], o32.displ, o64.displ), (te, fte)
+        assert _close(f["pot"], o32.get(oracle.POT), o64.get(oracle.POT)), (te, fte)
+        s.close()

@@ -64,3 +64,15 @@ def test_kernel_maxima_match_ref_kernel(runs):
     got_ac = dict(rho=rac.max(), kappa=kac.max(), rhop=(rac + kac).max(), alpha=(np.float32(2.0) * kac).max())
     for name, v in log["acoustic_kernel_max"].items():
         assert float(got_ac[name]) == pytest.approx(v, rel=2e-5), name
+
+
+@pytest.mark.parametrize("tile_elems", [5, 33, 128])
+def test_kernels_in_tiles_of_other_sizes(runs, tile_elems):
+    from specfem2d_b200.coupled import coupled_kernels
+
+    db, ref, _, _, o32, o64 = runs
+    adj = np.zeros((1, db.nstep, 2))
+    adj[0, :, 0] = ref["adj_source"].astype(np.float32)
+    got = coupled_kernels(db, adj, checkpoint_every=400, tile_elems=tile_elems)
+    for name in ("rho", "kappa", "mu", "rho_ac", "kappa_ac"):
+        assert _close(got[name], o32[name], o64[name]), name

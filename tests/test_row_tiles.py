@@ -50,10 +50,10 @@ def _db(physics, nstep):
     if physics.endswith(("mixed", "point")):
         # coefficients that differ inside the elements: two sets, which points
         # name, or 24,000, which are more than are shared
-        f = np.arange(25).reshape(5, 5) % 2 + np.zeros(db.ibool.shape)
+        f, keys = np.arange(25).reshape(5, 5) % 2 + np.zeros(db.ibool.shape), ("a1", "b1", "a2", "b2", "phi1", "phi2")
         if physics.endswith("point"):
-            f = np.random.default_rng(4).uniform(0.0, 50.0, db.ibool.shape)
-        for k in ("b1", "b2", "phi1", "phi2"):
+            f, keys = np.random.default_rng(4).uniform(0.0, 50.0, db.ibool.shape), ("b1", "b2", "phi1", "phi2")
+        for k in keys:
             db.atten[k] = (db.atten[k] * (1.0 + 1e-3 * f)[..., None]).astype(np.float32)
     if physics == "aniso":
         f32 = np.float32
@@ -95,9 +95,19 @@ def test_lane_kernels_on_a_mesh_without_orientation(physics, tile_elems):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("physics,tile_elems", [("iso", 0), ("iso", 33), ("iso", 128), ("visco", 0), ("visco", 64),
-                                                ("visco", 128), ("visco point", 32)])
-def test_lane_gradient_on_a_mesh_without_orientation(physics, tile_elems):
+@pytest.mark.parametrize("physics", ["iso", "visco"])
+def test_lane_gradient_on_a_mesh_without_orientation(physics):
+    _lane_gradient(physics, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("physics,tile_elems", [("iso", 33), ("iso", 128), ("visco", 64), ("visco", 128),
+                                                ("visco point", 32)])
+def test_lane_gradient_in_larger_tiles(physics, tile_elems):
+    _lane_gradient(physics, tile_elems)
+
+
+def _lane_gradient(physics, tile_elems):
     import oracle
     from specfem2d_b200.fwi import FWIGradient
 
